@@ -17,7 +17,9 @@
 #include <cstdlib>
 #include <cstring>
 #include <map>
+#include <functional>
 #include <mutex>
+#include <queue>
 #include <string>
 #include <tuple>
 #include <type_traits>
@@ -895,25 +897,62 @@ int run_uneven(fomo_ctx* ctx, float dh, float dt, int nt, int nbc, int fd_order,
       if (r != CUDA_SUCCESS) return fail(ctx, FOMO_ECUDA, "uneven sweep: tensor map encoding failed");
     }
     // Strips in order of decreasing height (the longest segments first, a
-    // shot's strips side by side so that neighbours share halo rows in L2); the
-    // last wave of strips is cut into four z chunks (chunk-major) so that the
-    // persistent CTAs finish together.
+    // shot's strips side by side so that neighbours share halo rows in L2), cut
+    // in z where that shortens the step.  A segment costs its rows plus the
+    // D + N + 4 rows its pipeline takes to fill and drain; the cut is the one of
+    // shortest makespan when the resident CTAs take the segments in list order.
+    // Height 0 keeps whole strips and cuts only the last wave into four (chunk-major):
+    // large batches (64 shots: ~600 strips for 296 CTAs) stay with it or a near cut,
+    // small ones need the cuts to have work for every SM (16 shots of 200..2000 x
+    // 200..800: about 130 whole strips, one per SM, 383 us per step; cut, 122 us).
     std::vector<int> order(ns);
     for (int s = 0; s < ns; ++s) order[s] = s;
     std::stable_sort(order.begin(), order.end(),
                      [&](int a, int b) { return tab[a].nz > tab[b].nz; });
-    for (int s : order)
-      for (int x0 = 0; x0 < tab[s].nx; x0 += f.txo) sg.push_back(make_int4(s, x0, 0, tab[s].nz));
-    a_grid = std::min<int>(f.resident, (int)sg.size());
-    const int L = std::min<int>(a_grid, (int)sg.size());
-    std::vector<int4> tail(sg.end() - L, sg.end());
-    sg.resize(sg.size() - L);
-    for (int k2 = 0; k2 < 4; ++k2)
-      for (const int4& e : tail) {
-        const int za = (int)((long long)e.w * k2 / 4), zb = (int)((long long)e.w * (k2 + 1) / 4);
-        if (zb > za) sg.push_back(make_int4(e.x, e.y, za, zb));
+    auto cut = [&](int height, std::vector<int4>& out) {
+      out.clear();
+      for (int s : order) {
+        const int nz = tab[s].nz, n = height ? std::max(1, (nz + height / 2) / height) : 1;
+        for (int k2 = 0; k2 < n; ++k2) {
+          const int za = (int)((long long)nz * k2 / n), zb = (int)((long long)nz * (k2 + 1) / n);
+          for (int x0 = 0; x0 < tab[s].nx; x0 += f.txo) out.push_back(make_int4(s, x0, za, zb));
+        }
       }
-    if ((long long)sg.size() > max_seg) return fail(ctx, FOMO_ECUDA, "uneven sweep: segment table");
+      if (height) return;
+      const int L = std::min<int>(f.resident, (int)out.size());
+      const std::vector<int4> tail(out.end() - L, out.end());
+      out.resize(out.size() - L);
+      for (int k2 = 0; k2 < 4; ++k2)
+        for (const int4& e : tail) {
+          const int za = (int)((long long)e.w * k2 / 4), zb = (int)((long long)e.w * (k2 + 1) / 4);
+          if (zb > za) out.push_back(make_int4(e.x, e.y, za, zb));
+        }
+    };
+    auto makespan = [&](const std::vector<int4>& segs) {
+      std::priority_queue<long long, std::vector<long long>, std::greater<long long>> free_at;
+      for (int k2 = 0; k2 < f.resident; ++k2) free_at.push(0);
+      long long end = 0;
+      for (const int4& e : segs) {
+        const long long t = free_at.top() + (e.w - e.z) + std::max(N + 2, 5) + N + 4;
+        free_at.pop();
+        free_at.push(t);
+        end = std::max(end, t);
+      }
+      return end;
+    };
+    long long best = -1;
+    for (int height : {0, 512, 384, 256, 192, 128, 96, 64, 48, 32}) {
+      std::vector<int4> cand;
+      cut(height, cand);
+      if ((long long)cand.size() > max_seg) continue;
+      const long long m = makespan(cand);
+      if (best < 0 || m < best) {
+        best = m;
+        sg.swap(cand);
+      }
+    }
+    a_grid = std::min<int>(f.resident, (int)sg.size());
+    if (best < 0) return fail(ctx, FOMO_ECUDA, "uneven sweep: segment table");
     a_nseg = (int)sg.size();
     FOMO_CU(ctx, cudaMemcpyAsync(d_ashot, at.data(), sizeof(AcShot) * ns, cudaMemcpyHostToDevice, st));
     FOMO_CU(ctx, cudaMemcpyAsync(d_maps, mh.data(), sizeof(CUtensorMap) * mh.size(),
