@@ -154,22 +154,30 @@ struct TuneVal {
 std::mutex g_tune_mu;
 std::map<TuneKey, TuneVal> g_tune;
 
+// The variant FOMO_SWEEP_CONFIG names, or -1.
+int pinned_sweep_variant() {
+  const char* env = std::getenv("FOMO_SWEEP_CONFIG");
+  int v = -1;
+  return env && std::sscanf(env, "%d", &v) == 1 ? v : -1;
+}
+
+// pair16: only the shot-pair variant of binary16 values.
 // sets16 / o16: the binary16 arrays (set-major, sweep field order) and the
 // binary16 outputs of set 1 for the binary16 storage form; null for FP32.
 template <class FieldFn>
 int tune_sweep(fomo_ctx* ctx, cudaStream_t st, SweepPlan& sp, int N, const Geo2& g, int ns,
                float* const sets[2][5], const Coef& c, float dtx, float dtz, const HabcDev& h,
-               const ElMat& m, FieldFn field, long long* d_bounds, __half* const* sets16 = nullptr,
-               const ElOut16* o16 = nullptr) {
+               const ElMat& m, FieldFn field, long long* d_bounds, bool pair16,
+               __half* const* sets16 = nullptr, const ElOut16* o16 = nullptr) {
   const bool h16 = sets16 != nullptr;
-  const TuneKey key{N, g.nx, g.nz, ns, h16 ? 1 : 0};
+  const TuneKey key{N, g.nx, g.nz, ns, pair16 ? 2 : (h16 ? 1 : 0)};
   // FOMO_SWEEP_CONFIG="variant,TX,ctas_per_sm" pins the configuration (tests, sweeps)
   if (const char* env = std::getenv("FOMO_SWEEP_CONFIG")) {
     int v = 0, tx = 0, per_sm = 0;
     float fw = kFrameWeight;
     const int nr = std::sscanf(env, "%d,%d,%d,%f", &v, &tx, &per_sm, &fw);
     if (nr >= 3 && v >= 0 && v < sweep_num_variants() && per_sm >= 1) {
-      if (sweep_variant_h16(v) != h16)
+      if (sweep_variant_h16(v) != h16 || sweep_variant_pair16(v) != pair16)
         return fail(ctx, FOMO_EARG, "FOMO_SWEEP_CONFIG names a variant of the other storage form");
       FOMO_CU(ctx, make_sweep_plan(sp, N, v, tx, per_sm, g, ns, sets, fw, d_bounds, st, sets16));
       return FOMO_OK;
@@ -207,7 +215,7 @@ int tune_sweep(fomo_ctx* ctx, cudaStream_t st, SweepPlan& sp, int N, const Geo2&
   // on every problem; FOMO_SWEEP_CONFIG still selects them).
   const bool pairs_ok = !h16 && m.ppack != nullptr && ns >= 2;
   for (int v = 0; v < sweep_num_variants(); ++v) {
-    if (sweep_variant_h16(v) != h16) continue;
+    if (sweep_variant_h16(v) != h16 || sweep_variant_pair16(v) != pair16) continue;
     if (sweep_variant_pair(v) ? !pairs_ok : !sweep_variant_ws(v)) continue;
     int txs[4];
     int ntx = sweep_tx_candidates(v, N, g.nx, txs, 4);
@@ -333,13 +341,20 @@ int run2d(fomo_ctx* ctx, Plan2& P, const float* vp, const float* vs, const float
   // shot-pair sweep, whose pair-interleaved fields hold an even number of shots
   // (an odd batch carries one all-zero shot).
   const bool sweep = kernel == FOMO_KERNEL_SINGLE_SWEEP;
-  const bool pair_ok = sweep && !P.fp16 && P.phys == kElastic;
+  // Binary16 batches of two or more shots run the shot-pair sweep's variant of
+  // binary16 values in FP32 words (same results, and less memory than a binary16
+  // array beside the FP32 band array: 4 bytes per stored value instead of 6);
+  // single shots and a pinned one-shot variant keep binary16 arrays (`half`).
+  const int pinv = pinned_sweep_variant();
+  const bool pair16 = sweep && P.fp16 && P.ns >= 2 && (pinv < 0 || sweep_variant_pair16(pinv));
+  const bool half = P.fp16 && !pair16;
+  const bool pair_ok = sweep && !half && P.phys == kElastic;
   const int nsa = pair_ok ? P.ns + (P.ns & 1) : P.ns;
   Arena ar;
   size_t o_model = P.dev ? 0 : ar.take<float>(3 * nint);
   size_t o_mat = ar.take<float>(nmat * P.plane);
   size_t o_state = ar.take<float>((long long)nsets * nfield * nsa * P.plane);
-  size_t o_state16 = P.fp16 ? ar.take<__half>((long long)nsets * nfield * P.ns * P.plane) : 0;
+  size_t o_state16 = half ? ar.take<__half>((long long)nsets * nfield * P.ns * P.plane) : 0;
   size_t o_unpack = ((P.fp16 || pair_ok) && opts && opts->final_state)
                         ? ar.take<float>(P.nxp * (long long)P.nzp)
                         : 0;
@@ -403,7 +418,7 @@ int run2d(fomo_ctx* ctx, Plan2& P, const float* vp, const float* vs, const float
   }
   float* d_mat = ws_ptr<float>(ctx, o_mat);
   float* d_state = ws_ptr<float>(ctx, o_state);
-  __half* d_state16 = P.fp16 ? ws_ptr<__half>(ctx, o_state16) : nullptr;
+  __half* d_state16 = half ? ws_ptr<__half>(ctx, o_state16) : nullptr;
   float* d_w = ws_ptr<float>(ctx, o_w);
   int32_t* d_src = ws_ptr<int32_t>(ctx, o_src);
   int32_t* d_rec = ws_ptr<int32_t>(ctx, o_rec);
@@ -428,8 +443,9 @@ int run2d(fomo_ctx* ctx, Plan2& P, const float* vp, const float* vs, const float
                                d_mat + 2 * P.plane, d_mat + 3 * P.plane, d_mat + 4 * P.plane));
   // ---- zero state (reset!, batch.jl:30-35) ----
   FOMO_CU(ctx, cudaMemsetAsync(d_state, 0, sizeof(float) * nsets * nfield * nsa * P.plane, st));
-  if (P.fp16) {
+  if (half)
     FOMO_CU(ctx, cudaMemsetAsync(d_state16, 0, sizeof(__half) * nsets * nfield * P.ns * P.plane, st));
+  if (P.fp16) {
     // fold the storage scales into the materials (powers of two: exact)
     k_scale<<<256, 256, 0, st>>>(d_mat, 2 * P.plane, kFp16Sv / kFp16St);
     k_scale<<<256, 256, 0, st>>>(d_mat + 2 * P.plane, 3 * P.plane, kFp16St / kFp16Sv);
@@ -490,7 +506,7 @@ int run2d(fomo_ctx* ctx, Plan2& P, const float* vp, const float* vs, const float
                          {field(1, 2), field(1, 3), field(1, 4), field(1, 0), field(1, 1)}};
     __half* sets16[10];
     ElOut16 o16{};
-    if (P.fp16) {
+    if (half) {
       const int order[5] = {2, 3, 4, 0, 1};  // txx, tzz, txz, vx, vz
       for (int s2 = 0; s2 < 2; ++s2)
         for (int f = 0; f < 5; ++f) sets16[s2 * 5 + f] = hfield(s2, order[f]).f16;
@@ -499,12 +515,12 @@ int run2d(fomo_ctx* ctx, Plan2& P, const float* vp, const float* vs, const float
     }
     rc = tune_sweep(ctx, st, sp, P.N, g, P.ns, sets, c, dtx, dtz, h, emat,
                     [&](int set, int f) { return field(set, f); },
-                    ws_ptr<long long>(ctx, o_bounds), P.fp16 ? sets16 : nullptr,
-                    P.fp16 ? &o16 : nullptr);
+                    ws_ptr<long long>(ctx, o_bounds), pair16, half ? sets16 : nullptr,
+                    half ? &o16 : nullptr);
     if (rc) return rc;
     // the tuning launches ran on the zero state; restore it
     FOMO_CU(ctx, cudaMemsetAsync(d_state, 0, sizeof(float) * nsets * nfield * nsa * P.plane, st));
-    if (P.fp16)
+    if (half)
       FOMO_CU(ctx, cudaMemsetAsync(d_state16, 0, sizeof(__half) * nsets * nfield * P.ns * P.plane,
                                    st));
   }
@@ -833,14 +849,14 @@ int run2d(fomo_ctx* ctx, Plan2& P, const float* vp, const float* vs, const float
     } else if (P.phys == kElastic) {
       ElFields a{field(A, 0), field(A, 1), field(A, 2), field(A, 3), field(A, 4)};
       const ElMat& m = emat;
-      if (P.fp16 && kernel == FOMO_KERNEL_SINGLE_SWEEP) {
+      if (half && kernel == FOMO_KERNEL_SINGLE_SWEEP) {
         ElOut o{field(B, 0), field(B, 1), field(B, 2), field(B, 3), field(B, 4)};
         const ElOut16 o16{hfield(B, 0).f16, hfield(B, 1).f16, hfield(B, 2).f16, hfield(B, 3).f16,
                           hfield(B, 4).f16};
         FOMO_CU(ctx, launch_sweep_elastic(st, sp, A, c, dtx, dtz, h, a, m, o, ctx->d_flag, &o16));
         launches += 1;
         sweeps_per_step = 1;
-      } else if (P.fp16) {
+      } else if (half) {
         HSet ha{{hfield(A, 0), hfield(A, 1), hfield(A, 2), hfield(A, 3), hfield(A, 4)}};
 #define FOMO_ELH_CASE(NN)                                                                       \
   case NN:                                                                                      \
@@ -863,12 +879,12 @@ int run2d(fomo_ctx* ctx, Plan2& P, const float* vp, const float* vs, const float
         sweeps_per_step = 2;
       }
       FOMO_CU(ctx, prof_mark(it, 1));
-      if (P.fp16)
+      if (half)
         k_elh_inject_record<<<P.ns, 256, 0, st>>>(it, P.nt, g, P.n_src, d_src, d_wav, hfield(B, 2),
                                                   hfield(B, 3), P.n_rec, d_rec, hfield(B, 0),
                                                   hfield(B, 1), d_seis[0], d_seis[1]);
       else if (pairs)
-        FOMO_CU(ctx, launch_inject_record_pair(st, it, P.nt, P.ns, P.plane, P.n_src, d_src, d_wav,
+        FOMO_CU(ctx, launch_inject_record_pair(st, pair16, g, it, P.nt, P.ns, P.n_src, d_src, d_wav,
                                                field(B, 2), field(B, 3), P.n_rec, d_rec,
                                                field(B, 0), field(B, 1), d_seis[0], d_seis[1]));
       else if (!tagged)
@@ -918,14 +934,14 @@ int run2d(fomo_ctx* ctx, Plan2& P, const float* vp, const float* vs, const float
     }
     FOMO_CU(ctx, cudaGetLastError());
     // snapshot of the interior (fused_kernels.jl:192-195): p (acoustic), vz (elastic)
-    if (P.fp16 && d_snap && P.snap_interval > 0 && it % P.snap_interval == 0) {
+    if (half && d_snap && P.snap_interval > 0 && it % P.snap_interval == 0) {
       const int k = it / P.snap_interval - 1;
       k_elh_unpack<<<dim3(cdiv(P.nx, 128), P.nz), 128, 0, st>>>(
           g, hfield(B, 1), 0, P.pad, P.pad, P.nx, P.nz, kFp16Sv, d_snap + (long long)k * nint);
     } else if (pairs && d_snap && P.snap_interval > 0 && it % P.snap_interval == 0) {
       const int k = it / P.snap_interval - 1;  // vz of shot 0, interior
       FOMO_CU(ctx, launch_pair_unpack(st, field(B, 1), P.plane, P.ld, P.pad, P.pad, P.nx, P.nz, 0,
-                                      d_snap + (long long)k * nint));
+                                      pair16 ? kFp16Sv : 1.0f, d_snap + (long long)k * nint));
     } else if (d_snap && P.snap_interval > 0 && it % P.snap_interval == 0) {
       int k = it / P.snap_interval - 1;
       const float* src = (P.phys == kAcoustic ? field(B, 2) : field(replica ? A : B, 1)) + P.pad +
@@ -998,7 +1014,7 @@ int run2d(fomo_ctx* ctx, Plan2& P, const float* vp, const float* vs, const float
     const long long hp = (long long)P.nxp * P.nzp;
     for (int s = 0; s < P.ns; ++s)
       for (int f = 0; f < (P.phys == kScalar ? 2 : nfield); ++f) {
-        if (P.fp16) {  // unscaled FP32 copy of the stored field
+        if (half) {  // unscaled FP32 copy of the stored field
           float* tmp = ws_ptr<float>(ctx, o_unpack);
           k_elh_unpack<<<dim3(cdiv(P.nxp, 128), P.nzp), 128, 0, st>>>(
               g, hfield(A, f), (long long)s * P.plane, 0, 0, P.nxp, P.nzp,
@@ -1011,7 +1027,7 @@ int run2d(fomo_ctx* ctx, Plan2& P, const float* vp, const float* vs, const float
         if (pairs) {
           float* tmp = ws_ptr<float>(ctx, o_unpack);
           FOMO_CU(ctx, launch_pair_unpack(st, field(A, f), P.plane, P.ld, 0, 0, P.nxp, P.nzp, s,
-                                          tmp));
+                                          !pair16 ? 1.0f : (f < 2 ? kFp16Sv : kFp16St), tmp));
           FOMO_CU(ctx, cudaMemcpyAsync(opts->final_state + ((long long)s * nfield + f) * hp, tmp,
                                        sizeof(float) * hp, cudaMemcpyDeviceToHost, st));
           FOMO_CU(ctx, cudaStreamSynchronize(st));  // tmp is reused by the next field
@@ -1050,7 +1066,7 @@ int run2d(fomo_ctx* ctx, Plan2& P, const float* vp, const float* vs, const float
     double wpc = P.phys == kElastic ? 10.0 : (P.phys == kAcoustic ? 6.0 : 3.0);
     double wm = P.phys == kElastic ? 5.0 : (P.phys == kAcoustic ? 3.0 : 1.0);
     double wbytes = 4.0;  // bytes of a stored wavefield word
-    if (P.fp16) {         // binary16 outside the FP32 band
+    if (half) {           // binary16 outside the FP32 band
       const double inner = (double)std::max(0, P.nxp - 2 * kFp16Band) * std::max(0, P.nzp - 2 * kFp16Band);
       wbytes = (4.0 * (cells - inner) + 2.0 * inner) / cells;
     }

@@ -2736,6 +2736,10 @@ bool sweep_variant_pair(int variant) {
   return variant >= kPairBase && variant < kPairBase + pair_num_variants();
 }
 
+bool sweep_variant_pair16(int variant) {
+  return sweep_variant_pair(variant) && pair_variant16(variant - kPairBase);
+}
+
 int sweep_pack_pitch(int nx) { return ((nx + 2 * 128 + kPackColPad) / 2 + 16) & ~15; }
 
 size_t sweep_pack_floats(int nx, int nz) {

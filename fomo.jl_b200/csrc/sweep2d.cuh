@@ -102,6 +102,7 @@ struct PairCoef {
   float2 nq, nqt, nqxt;  // -q, -qt, -qxt
 };
 int pair_num_variants();
+bool pair_variant16(int v);  // the variant of binary16 values in FP32 words
 int pair_threads(int v);
 int pair_txmax(int N, int v);       // widest strip of a variant (even)
 int pair_box_width(int N, int v);   // TMA box width in float2 elements
@@ -116,17 +117,20 @@ cudaError_t launch_pair_elastic(cudaStream_t st, const SweepPlan& sp, int v, int
                                 const PairCoef& k, const HabcDev& h, const PairPack& mp,
                                 const PairOut& o, int* err);
 // Injection then recording of one step on pair-layout txx/tzz and vx/vz
-// (k_inject_record's order and semantics), one block per shot.
-cudaError_t launch_inject_record_pair(cudaStream_t st, int it, int nt, int ns, long long plane,
-                                      int n_src, const int* src_lin, const float* wav, float* txx,
-                                      float* tzz, int n_rec, const int* rec_lin, const float* vx,
-                                      const float* vz, float* s0, float* s1);
+// (k_inject_record's order and semantics; h16: k_elh_inject_record's), one
+// block per shot.
+cudaError_t launch_inject_record_pair(cudaStream_t st, bool h16, const Geo2& g, int it, int nt,
+                                      int ns, int n_src, const int* src_lin, const float* wav,
+                                      float* txx, float* tzz, int n_rec, const int* rec_lin,
+                                      const float* vx, const float* vz, float* s0, float* s1);
 // Columns [x0, x0 + nx) of rows [z0, z0 + nz) of shot `shot` of a pair-layout
-// field into out (unpitched).
+// field over `scale` into out (unpitched).
 cudaError_t launch_pair_unpack(cudaStream_t st, const float* f, long long plane, int ld, int x0,
-                               int z0, int nx, int nz, int shot, float* out);
-// Is a sweep variant (the plan numbering) a shot-pair / warp-specialized variant?
+                               int z0, int nx, int nz, int shot, float scale, float* out);
+// Is a sweep variant (the plan numbering) a shot-pair / warp-specialized variant,
+// or the shot-pair variant of binary16 values?
 bool sweep_variant_pair(int variant);
+bool sweep_variant_pair16(int variant);
 bool sweep_variant_ws(int variant);
 
 // Kernel family for a problem (FOMO_KERNEL_TWO_PHASE / _SINGLE_SWEEP).

@@ -67,6 +67,12 @@ __device__ __forceinline__ float2 ph_corner(const float4& wt, float2 fc, float2 
   return p_fma(lo2(wt), fc, p_mul(p_mul(hi2(wt), make_float2(0.5f, 0.5f)), p_add(sx, sz)));
 }
 
+// Both lanes rounded to binary16 (nearest even) and widened again: one packed
+// conversion down, two up.
+__device__ __forceinline__ float2 p_round16(float2 v) {
+  return __half22float2(__float22half2_rn(v));
+}
+
 // The value as the result of an (empty) asm statement: the compiler keeps a
 // duplicated constant pair in registers instead of rebuilding it from the
 // constant bank before every packed instruction that reads it.
@@ -106,7 +112,15 @@ struct PairShape {
   static_assert((2 * W * 8) % 128 == 0, "two-row boxes keep 128-byte alignment");
 };
 
-template <int N, int NV, int P, int MINB>
+// H16: precision = fp16.  Every stored value outside the FP32 band is rounded
+// to binary16 before it is used or stored (the velocities before the stress
+// update reads them), as the binary16 forms store it; the fields keep the
+// rounded values in FP32 words.  This kernel is bound by issue at about a third of the
+// HBM bandwidth, so halving the words gains nothing, while binary16 words
+// cost a conversion per stencil operand: rounding the five results per cell
+// instead takes 0.242 ms per step against 0.688 ms per step for the one-shot binary16 sweep
+// (16 shots of 1000 x 500, order 10, nbc 80).
+template <int N, int NV, int P, int MINB, bool H16>
 __global__ void __launch_bounds__(2 * NV, MINB)
     k_el_pair(const __grid_constant__ CUtensorMap tm_xx, const __grid_constant__ CUtensorMap tm_zz,
               const __grid_constant__ CUtensorMap tm_xz, const __grid_constant__ CUtensorMap tm_vx,
@@ -332,6 +346,11 @@ __global__ void __launch_bounds__(2 * NV, MINB)
                 }
               }
             }
+            if constexpr (H16)
+              if (g.xds >= kFp16Band && zdist(qv) >= kFp16Band) {
+                vv[0] = p_round16(vv[0]);
+                vv[1] = p_round16(vv[1]);
+              }
             const int vr = ring(vw, rr, LVV);  // v'' ring row of qv
             s_vv[vr * W + c] = vv[0];
             s_vv[(LVV + vr) * W + c] = vv[1];
@@ -494,6 +513,11 @@ __global__ void __launch_bounds__(2 * NV, MINB)
                 }
               }
             }
+            if constexpr (H16)
+              if (g.xds >= kFp16Band && zdist(qs) >= kFp16Band) {
+#pragma unroll
+                for (int f = 0; f < 3; ++f) v[f] = p_round16(v[f]);
+              }
             const long long d = rr ? gm.ld : 0;
             ot0[d] = v[0];
             ot1[d] = v[1];
@@ -528,26 +552,26 @@ __global__ void __launch_bounds__(2 * NV, MINB)
 
 namespace {
 
-// Pair variants: (form 0; threads per role; TMA prefetch depth in row pairs;
+// Pair variants: (form: 0 FP32, 1 binary16 values; threads per role; TMA prefetch depth in row pairs;
 // CTAs per SM the register budget targets).  Deeper prefetch keeps more HBM
 // reads in flight per SM; narrower CTAs keep two or three of them resident.
 #define FOMO_PAIR_VARIANTS(X, NN)                                                         \
   X(0, NN, 0, 128, 1, 2) X(1, NN, 0, 96, 2, 2) X(2, NN, 0, 96, 3, 2) X(3, NN, 0, 64, 3, 3) \
-  X(4, NN, 0, 128, 3, 1)
-constexpr int kPairNV[] = {128, 96, 96, 64, 128};
+  X(4, NN, 0, 128, 3, 1) X(5, NN, 1, 128, 1, 2)
+constexpr int kPairNV[] = {128, 96, 96, 64, 128, 128};
+constexpr int kPair16 = 5;  // the variant of binary16 values
 constexpr int kNumPair = sizeof(kPairNV) / sizeof(kPairNV[0]);
 constexpr int kMaxDynSmemPair = 227 * 1024;
 
 template <int N, int F, int NV, int P>
 size_t pair_smem_bytes(int wstride) {
-  static_assert(F == 0, "one kernel form");
   using S = PairShape<N, NV, P>;
   return (size_t)S::O_WT * 8 + (size_t)3 * wstride * 16 + sizeof(uint64_t) * S::NO;
 }
 
 template <int N, int F, int NV, int P, int MINB>
 auto pair_kernel() {
-  return k_el_pair<N, NV, P, MINB>;
+  return k_el_pair<N, NV, P, MINB, F == 1>;
 }
 
 template <int N, int F, int NV, int P, int MINB>
@@ -599,48 +623,63 @@ __global__ void k_pair_pack(int nx, int nz, int ld, ElMat m, float4* pv, float4*
 
 // Injection then recording on the pair layout, one block per shot (the
 // semantics of k_inject_record: sources added in source order by one thread,
-// then the receivers sampled after the barrier).
-__global__ void k_inject_record_pair(int it, int nt, long long plane, int n_src,
+// then the receivers sampled after the barrier).  H16: scaled fields of
+// binary16 values outside the band (k_elh_inject_record's semantics).
+template <bool H16>
+__global__ void k_inject_record_pair(Geo2 g, int it, int nt, long long plane, int n_src,
                                      const int* __restrict__ src_lin,
                                      const float* __restrict__ wav, float* txx, float* tzz,
                                      int n_rec, const int* __restrict__ rec_lin,
                                      const float* vx, const float* vz, float* __restrict__ s0,
                                      float* __restrict__ s1) {
   const int s = blockIdx.x;
+  const float sv = H16 ? kFp16Sv : 1.0f;  // powers of two: exact
   const long long so = (long long)(s >> 1) * 2 * plane + (s & 1);
   if (threadIdx.x == 0) {
     for (int q = 0; q < n_src; ++q) {
-      const long long p = so + 2LL * src_lin[(long long)s * n_src + q];
-      const float w = wav[(long long)(it - 1) * n_src + q];
-      txx[p] = __fadd_rn(txx[p], w);
-      tzz[p] = __fadd_rn(tzz[p], w);
+      const int cell = src_lin[(long long)s * n_src + q];
+      const long long p = so + 2LL * cell;
+      float w = wav[(long long)(it - 1) * n_src + q];
+      if constexpr (H16) w = __fmul_rn(w, kFp16St);
+      float a = __fadd_rn(txx[p], w), b = __fadd_rn(tzz[p], w);
+      if constexpr (H16) {
+        const int x = cell % g.ld, z = cell / g.ld;
+        if (min(min(x, g.nx - 1 - x), min(z, g.nz - 1 - z)) >= kFp16Band) {
+          a = __half2float(__float2half_rn(a));
+          b = __half2float(__float2half_rn(b));
+        }
+      }
+      txx[p] = a;
+      tzz[p] = b;
     }
   }
   __syncthreads();
   const long long ob = (long long)n_rec * ((long long)(it - 1) + (long long)nt * s);
   for (int r = threadIdx.x; r < n_rec; r += blockDim.x) {
     const long long p = so + 2LL * rec_lin[r];
-    if (s0) s0[ob + r] = vx[p];
-    if (s1) s1[ob + r] = vz[p];
+    if (s0) s0[ob + r] = H16 ? __fdiv_rn(vx[p], sv) : vx[p];
+    if (s1) s1[ob + r] = H16 ? __fdiv_rn(vz[p], sv) : vz[p];
   }
 }
 
 // Columns [x0, x0 + nx) of rows [z0, z0 + nz) of one shot of a pair-layout
-// field, unpitched.
+// field divided by its storage scale (a power of two: exact), unpitched.
 __global__ void k_pair_unpack(const float* __restrict__ f, long long plane, int ld, int x0, int z0,
-                              int nx, int nz, int shot, float* __restrict__ out) {
+                              int nx, int nz, int shot, float scale, float* __restrict__ out) {
   const long long n = (long long)nx * nz;
   const long long so = (long long)(shot >> 1) * 2 * plane + (shot & 1);
   for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < n;
        q += (long long)gridDim.x * blockDim.x) {
     const long long z = q / nx, x = q - z * nx;
-    out[q] = f[so + 2 * ((z + z0) * ld + x + x0)];
+    out[q] = __fdiv_rn(f[so + 2 * ((z + z0) * ld + x + x0)], scale);
   }
 }
 
 }  // namespace
 
 int pair_num_variants() { return kNumPair; }
+
+bool pair_variant16(int v) { return v == kPair16; }
 
 int pair_threads(int v) { return v >= 0 && v < kNumPair ? 2 * kPairNV[v] : 0; }
 
@@ -731,18 +770,19 @@ cudaError_t launch_pair_elastic(cudaStream_t st, const SweepPlan& sp, int v, int
   return cudaErrorInvalidValue;
 }
 
-cudaError_t launch_inject_record_pair(cudaStream_t st, int it, int nt, int ns, long long plane,
-                                      int n_src, const int* src_lin, const float* wav, float* txx,
-                                      float* tzz, int n_rec, const int* rec_lin, const float* vx,
-                                      const float* vz, float* s0, float* s1) {
-  k_inject_record_pair<<<ns, 256, 0, st>>>(it, nt, plane, n_src, src_lin, wav, txx, tzz, n_rec,
-                                           rec_lin, vx, vz, s0, s1);
+cudaError_t launch_inject_record_pair(cudaStream_t st, bool h16, const Geo2& g, int it, int nt,
+                                      int ns, int n_src, const int* src_lin, const float* wav,
+                                      float* txx, float* tzz, int n_rec, const int* rec_lin,
+                                      const float* vx, const float* vz, float* s0, float* s1) {
+  auto kern = h16 ? k_inject_record_pair<true> : k_inject_record_pair<false>;
+  kern<<<ns, 256, 0, st>>>(g, it, nt, g.plane, n_src, src_lin, wav, txx, tzz, n_rec, rec_lin, vx,
+                           vz, s0, s1);
   return cudaGetLastError();
 }
 
 cudaError_t launch_pair_unpack(cudaStream_t st, const float* f, long long plane, int ld, int x0,
-                               int z0, int nx, int nz, int shot, float* out) {
-  k_pair_unpack<<<256, 256, 0, st>>>(f, plane, ld, x0, z0, nx, nz, shot, out);
+                               int z0, int nx, int nz, int shot, float scale, float* out) {
+  k_pair_unpack<<<256, 256, 0, st>>>(f, plane, ld, x0, z0, nx, nz, shot, scale, out);
   return cudaGetLastError();
 }
 
