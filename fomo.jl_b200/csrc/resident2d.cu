@@ -1,0 +1,104 @@
+// resident2d.cu -- tile plan of the on-chip 2D time loops (resident2d.cuh).
+#include <algorithm>
+#include <numeric>
+
+#include "resident2d.cuh"
+
+namespace fomo {
+namespace res {
+
+namespace {
+constexpr int kMaxSmem = 227 * 1024;
+int align4(int n) { return (n + 3) & ~3; }
+}  // namespace
+
+Plan make_plan(const Needs& nd, int N, int nx, int nz, int ld, int nbc, int ns, int nsm,
+               int extra) {
+  Plan best;
+  if (ns < 1 || ns > nsm) return best;
+  const int per = nsm / ns, H = N + 1, L = align4(N);
+  double best_cost = 0.0;
+  for (int gx = 1; gx <= per; ++gx) {
+    int TW = 0, narrow = nx, nq = 0;
+    for (int i = 0; i < gx; ++i) {
+      const int a = tile_x(nx, gx, i), b = tile_x(nx, gx, i + 1), first = a ? a - 1 : 0;
+      TW = std::max(TW, b - a);
+      narrow = std::min(narrow, b - a);
+      nq = std::max(nq, (std::min(b, nx - 1) - first) / 4 + 1);
+    }
+    if (gx > 1 && narrow < H) break;
+    const int gz = std::max(1, std::min(per / gx, nz / H));
+    for (int z = std::max(1, gz - 2); z <= gz; ++z) {
+      const int TH = (nz + z - 1) / z;
+      for (int form = 0; form < kNumForms; ++form) {
+        const int R = kForms[form].R, CX = kForms[form].CX, nb = 4 * nq / CX;
+        const int ngr = (TH + 2 + R - 1) / R, thr = nb * ngr;
+        if (thr > kForms[form].threads) continue;
+        const int rows = ngr * R + 2 * N + 1;
+        // columns: L + the quads + the right halo, padded so that the 16-byte reads
+        // of a warp that spans row groups miss each other's banks
+        const int need = L + 4 * nq + (N == 5 ? 8 : 4);
+        for (int pad = 28; pad >= 0; pad -= 4) {
+          const int pitch = need + pad;
+          if (pad && (R * (pitch / 4) - nq) % 8 != 0) continue;
+          const int floats = (nd.hal * rows * pitch +
+                              (nd.ext + (CX * R > nd.mreg ? nd.mats : 0)) * ngr * R * 4 * nq + extra + 3) &
+                             ~3;
+          // words put (4 bytes of table each) and got (8 bytes) by both half steps
+          const int put = (2 * N + 1 + nd.wide) * (nd.strips * TH + nd.bands * TW) +
+                          2 * (nd.rows * TW + nd.cols * TH);
+          const int get = put + 2 * (2 * N + 1 + nd.wide) * (nd.strips + nd.bands);
+          const size_t smem = sizeof(float) * floats + sizeof(int) * (put + 2) + sizeof(Word) * get;
+          if (smem > (size_t)kMaxSmem) continue;
+          // the slowest tile sets the pace: its extended cells, plus the halo it reads
+          const double cost = 4.0 * R * nq * ngr + form + 2.0 * (TW + TH) * (2 * N + 2) * 0.3;
+          if (best.ok && cost >= best_cost) continue;
+          best_cost = cost;
+          best.ok = true;
+          best.form = form;
+          // idle threads of a small tile still move words
+          best.threads = (std::min(kForms[form].threads, std::max(thr, get / 6)) + 31) & ~31;
+          best.tiles = gx * z * ns;
+          best.smem = smem;
+          best.g = Geom{nx, nz, ld, (long long)ld * nz, N, nbc, gx, z, nq, ngr, nb, pitch, rows, floats, put};
+        }
+      }
+    }
+  }
+  return best;
+}
+
+void plan_entries(Plan& p, int ns, const CellTagHost& tags) {
+  const Geom& g = p.g;
+  struct Item {
+    int tile, thread, cell, e;
+  };
+  std::vector<Item> items;
+  for (int e = 0; e < (int)tags.lin.size(); ++e) {
+    const int x = tags.lin[e] % g.ld, z = tags.lin[e] / g.ld;
+    int tx = 0, tz = 0;
+    while (tile_x(g.nx, g.gx, tx + 1) <= x) ++tx;
+    while (tile_z(g.nz, g.gz, tz + 1) <= z) ++tz;
+    const int x0 = tile_x(g.nx, g.gx, tx);
+    const int ex = x - (x0 ? x0 - 1 : 0), ez = z - tile_z(g.nz, g.gz, tz) + 1;  // extended
+    const Form f = kForms[p.form];
+    const int thread = (ez / f.R) * g.nb + ex / f.CX, cell = (ez % f.R) * f.CX + ex % f.CX;
+    for (int s = 0; s < ns; ++s)
+      items.push_back(Item{(s * g.gz + tz) * g.gx + tx, thread, cell, e});
+  }
+  std::stable_sort(items.begin(), items.end(), [](const Item& a, const Item& b) {
+    return a.tile != b.tile ? a.tile < b.tile : a.thread < b.thread;
+  });
+  p.off.assign(p.tiles + 1, 0);
+  p.key.resize(items.size());
+  p.ent.resize(items.size());
+  for (const Item& it : items) ++p.off[it.tile + 1];
+  std::partial_sum(p.off.begin(), p.off.end(), p.off.begin());
+  for (size_t k = 0; k < items.size(); ++k) {
+    p.key[k] = make_int2(items[k].thread, items[k].cell);
+    p.ent[k] = items[k].e;
+  }
+}
+
+}  // namespace res
+}  // namespace fomo

@@ -15,6 +15,7 @@
 #include "solver2d_kernels.cuh"
 #include "mixed2d.cuh"
 #include "replica2d.cuh"
+#include "resident2d.cuh"
 #include "sweep2d.cuh"
 
 namespace fomo {
@@ -262,6 +263,21 @@ int tune_sweep(fomo_ctx* ctx, cudaStream_t st, SweepPlan& sp, int N, const Geo2&
   return FOMO_OK;
 }
 
+// Runs of more steps than this keep their state on the chip when it fits: at every
+// size measured that halves the step (figures in resident2d.cuh).  Shorter runs gain
+// under 2 ms a call and keep the replayed launches, whose count callers read in the
+// stats and the tests pin.
+constexpr int kResMinSteps = 300;
+
+int sm_count(int device) {
+  int n = 0;
+  if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) {
+    cudaGetLastError();
+    return 0;
+  }
+  return n;
+}
+
 struct Outs {
   float* seis[3];
   int nseis;
@@ -374,15 +390,36 @@ int run2d(fomo_ctx* ctx, Plan2& P, const float* vp, const float* vs, const float
   // separate kernel: a step costs tens of microseconds there, and the tag code
   // raises the acoustic pressure kernel from 40 to 54 registers (6 -> 4 blocks
   // per SM).
-  const bool tagged = !P.fp16 && !hook && (long long)P.nxp * P.nzp * P.ns <= 2000000LL &&
+  //
+  // Runs whose state fits on the chip keep it there for the whole time loop
+  // (resident2d.cuh): AUTO's pick for more than kResMinSteps steps.
+  const bool prof_req = opts && (opts->flags & FOMO_F_PROFILE);
+  res::Plan rp;
+  if (P.kernel == FOMO_KERNEL_AUTO && kernel == FOMO_KERNEL_TWO_PHASE && !P.fp16 && !hook && !prof_req && P.nt > kResMinSteps &&
+      !(opts && (opts->flags & FOMO_F_STEP_LAUNCH)))
+    rp = res::make_plan(P.phys == kAcoustic  ? res::kAcousticNeeds
+                        : P.phys == kElastic ? res::kElasticNeeds
+                                             : res::kScalarNeeds,
+                        P.N, P.nxp,
+                        P.nzp, P.ld, hh.nbc, P.ns, sm_count(ctx->device),
+                        res::smem_extra(hh.wstride, P.sponge ? P.nbc : 0));
+  const bool tagged = !rp.ok && !P.fp16 && !hook && (long long)P.nxp * P.nzp * P.ns <= 2000000LL &&
                       (P.phys == kScalar || kernel == FOMO_KERNEL_TWO_PHASE);
   CellTagHost tags;
-  if (tagged) tags = make_cell_tags(src_lin.data(), (int)nsrc_all, rec_lin.data(), P.n_rec);
+  if (tagged || rp.ok)
+    tags = make_cell_tags(src_lin.data(), (int)nsrc_all, rec_lin.data(), P.n_rec);
   const int n_ent = (int)tags.lin.size();
   size_t o_tag = tagged ? ar.take<int32_t>(P.plane) : 0;
-  size_t o_ent = tagged ? ar.take<int4>(std::max(n_ent, 1)) : 0;
+  size_t o_ent = tagged || rp.ok ? ar.take<int4>(std::max(n_ent, 1)) : 0;
   size_t o_elin = tagged ? ar.take<int32_t>(std::max(n_ent, 1)) : 0;
-  size_t o_list = tagged ? ar.take<int32_t>(std::max<size_t>(tags.list.size(), 1)) : 0;
+  size_t o_list =
+      tagged || rp.ok ? ar.take<int32_t>(std::max<size_t>(tags.list.size(), 1)) : 0;
+  if (rp.ok) res::plan_entries(rp, P.ns, tags);
+  const size_t ll_words = rp.ok ? (size_t)4 * rp.tiles * rp.g.per : 0;
+  size_t o_ll = rp.ok ? ar.take<uint64_t>(ll_words) : 0;
+  size_t o_roff = rp.ok ? ar.take<int>(rp.off.size()) : 0;
+  size_t o_rkey = rp.ok ? ar.take<int2>(std::max<size_t>(rp.key.size(), 1)) : 0;
+  size_t o_rent = rp.ok ? ar.take<int>(std::max<size_t>(rp.ent.size(), 1)) : 0;
   size_t o_pack = sweep ? ar.take<float>(sweep_pack_floats(P.nxp, P.nzp)) : 0;
   size_t o_ppack = pair_ok ? ar.take<float>(pair_pack_floats(P.nxp, P.nzp)) : 0;
   // replica: strip backups of the five fields, three weight planes, frame scratch
@@ -461,15 +498,19 @@ int run2d(fomo_ctx* ctx, Plan2& P, const float* vp, const float* vs, const float
     int32_t* d_tag = ws_ptr<int32_t>(ctx, o_tag);
     FOMO_CU(ctx, cudaMemsetAsync(d_tag, 0xFF, sizeof(int32_t) * P.plane, st));  // -1
     if (n_ent) {
-      FOMO_CU(ctx, cudaMemcpyAsync(ws_ptr<int4>(ctx, o_ent), tags.ent.data(), sizeof(int4) * n_ent,
-                                   cudaMemcpyHostToDevice, st));
       FOMO_CU(ctx, cudaMemcpyAsync(ws_ptr<int32_t>(ctx, o_elin), tags.lin.data(),
                                    sizeof(int32_t) * n_ent, cudaMemcpyHostToDevice, st));
-      FOMO_CU(ctx, cudaMemcpyAsync(ws_ptr<int32_t>(ctx, o_list), tags.list.data(),
-                                   sizeof(int32_t) * tags.list.size(), cudaMemcpyHostToDevice, st));
       k_set_tags<<<cdiv(n_ent, 256), 256, 0, st>>>(d_tag, ws_ptr<int32_t>(ctx, o_elin), n_ent);
     }
     tg.tag = d_tag;
+  }
+  if (tagged || rp.ok) {
+    if (n_ent) {
+      FOMO_CU(ctx, cudaMemcpyAsync(ws_ptr<int4>(ctx, o_ent), tags.ent.data(), sizeof(int4) * n_ent,
+                                   cudaMemcpyHostToDevice, st));
+      FOMO_CU(ctx, cudaMemcpyAsync(ws_ptr<int32_t>(ctx, o_list), tags.list.data(),
+                                   sizeof(int32_t) * tags.list.size(), cudaMemcpyHostToDevice, st));
+    }
     tg.ent = ws_ptr<int4>(ctx, o_ent);
     tg.list = ws_ptr<int32_t>(ctx, o_list);
     tg.wav = d_wav;
@@ -675,7 +716,87 @@ int run2d(fomo_ctx* ctx, Plan2& P, const float* vp, const float* vs, const float
     }
     return e;
   };
-  {
+  // ---- the time loop on the chip ----
+  if (rp.ok) {
+    FOMO_CU(ctx, cudaMemcpyAsync(ws_ptr<int>(ctx, o_roff), rp.off.data(),
+                                 sizeof(int) * rp.off.size(), cudaMemcpyHostToDevice, st));
+    if (!rp.key.empty()) {
+      FOMO_CU(ctx, cudaMemcpyAsync(ws_ptr<int2>(ctx, o_rkey), rp.key.data(),
+                                   sizeof(int2) * rp.key.size(), cudaMemcpyHostToDevice, st));
+      FOMO_CU(ctx, cudaMemcpyAsync(ws_ptr<int>(ctx, o_rent), rp.ent.data(),
+                                   sizeof(int) * rp.ent.size(), cudaMemcpyHostToDevice, st));
+    }
+    res::Run run;
+    run.g = rp.g;
+    run.c = c;
+    run.dtx = dtx;
+    run.dtz = dtz;
+    run.h = h;
+    run.E = res::Entries{ws_ptr<int>(ctx, o_roff), ws_ptr<int2>(ctx, o_rkey),
+                         ws_ptr<int>(ctx, o_rent), tg};
+    run.ll = ws_ptr<uint64_t>(ctx, o_ll);
+    FOMO_CU(ctx, cudaMemsetAsync(run.ll, 0, sizeof(uint64_t) * ll_words, st));
+    run.snap_interval = d_snap ? P.snap_interval : 0;
+    run.pad = P.pad;
+    run.nxi = P.nx;
+    run.nzi = P.nz;
+    run.snaps = d_snap;
+    run.err = ctx->d_flag;
+    // one launch, or with host snapshots about eight, so that their frames are
+    // copied out while later steps run
+    const int si = run.snap_interval;
+    const bool stream = si && !P.dev && outs.snaps && P.nt >= 2 * si;
+    const int K = stream ? si * std::max(1, P.nt / (8 * si)) : P.nt;
+    const int nchunk = P.nt / K;
+    if (stream) {
+      chunk_ev.ev.assign(nchunk, nullptr);
+      for (auto& e : chunk_ev.ev) FOMO_CU(ctx, cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+      frames_per_chunk = K / si;
+    }
+    FOMO_CU(ctx, cudaEventRecord(ctx->ev0, st));  // the loop starts after the tables
+    bool first = true;
+    for (int it = 1; it <= P.nt; it += run.nsteps) {
+      run.it0 = it;
+      run.nsteps = std::min(K, P.nt - it + 1);
+      res::Fields f{};
+      for (int i = 0; i < nmat; ++i) f.mat[i] = d_mat + i * P.plane;
+      cudaError_t e;
+      if (P.phys == kScalar) {  // u^n in set B, u^{n-1} in set A; one launch, from zero
+        res::Centered cc{};
+        cc.c0 = 2.0f * kD2C0[P.N];
+        for (int l = 0; l < 5; ++l) cc.d2[l] = kD2[P.N][l];
+        f.out[0] = field(B, 0);
+        f.out[1] = field(A, 0);
+        e = res::launch_scalar(st, P.N, rp, run, f, cc);
+      } else {
+        for (int i = 0; i < nfield; ++i) {
+          f.in[i] = first ? nullptr : field(A, i);  // the run starts from zero
+          f.out[i] = field(B, i);
+        }
+        e = P.phys == kAcoustic ? res::launch_acoustic(st, P.N, P.sponge, rp, run, f)
+                                : res::launch_elastic(st, P.N, P.sponge, rp, run, f);
+      }
+      if (first && e == cudaErrorCooperativeLaunchTooLarge) {
+        cudaGetLastError();  // part of the SMs is not ours: launch the steps instead
+        rp.ok = false;
+        chunk_ev.ev.clear();
+        frames_per_chunk = 0;
+        break;
+      }
+      FOMO_CU(ctx, e);
+      first = false;
+      launches += 1;
+      if (P.phys != kScalar) std::swap(A, B);
+      const int k = it / K;
+      if (stream && run.nsteps == K) FOMO_CU(ctx, cudaEventRecord(chunk_ev.ev[k], st));
+    }
+    if (rp.ok) {
+      it_first = P.nt + 1;
+      sweeps_per_step = P.phys == kScalar ? 1 : 2;
+      if (stream) streamed_chunks = nchunk;
+    }
+  }
+  if (!rp.ok) {
     const bool scalar = P.phys == kScalar;
     const bool elastic = P.phys == kElastic;
     const bool chunks_ok = (!elastic || kernel == FOMO_KERNEL_TWO_PHASE) && !P.fp16 && !hook &&
@@ -1043,10 +1164,12 @@ int run2d(fomo_ctx* ctx, Plan2& P, const float* vp, const float* vs, const float
   FOMO_CU(ctx, cudaStreamSynchronize(st));
   if (streamed_chunks || lag_done || seis_done)
     FOMO_CU(ctx, cudaStreamSynchronize(ctx->copy_stream));
-  if (kernel == FOMO_KERNEL_SINGLE_SWEEP) {
+  if (kernel == FOMO_KERNEL_SINGLE_SWEEP || rp.ok) {
     int hflag = 0;
     FOMO_CU(ctx, cudaMemcpy(&hflag, ctx->d_flag, sizeof(int), cudaMemcpyDeviceToHost));
-    if (hflag) return fail(ctx, FOMO_ECUDA, "single-sweep kernel: a bounded TMA wait timed out");
+    if (hflag)
+      return fail(ctx, FOMO_ECUDA, rp.ok ? "on-chip time loop: a bounded halo wait timed out"
+                                         : "single-sweep kernel: a bounded TMA wait timed out");
   }
   float ms = 0.0f;
   FOMO_CU(ctx, cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1));
