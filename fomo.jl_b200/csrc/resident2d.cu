@@ -100,5 +100,43 @@ void plan_entries(Plan& p, int ns, const CellTagHost& tags) {
   }
 }
 
+Tables take_tables(Arena& ar, const Plan& p) {
+  Tables t;
+  if (!p.ok) return t;
+  t.ll_words = (size_t)4 * p.tiles * p.g.per;
+  t.ll = ar.take<uint64_t>(t.ll_words);
+  t.off = ar.take<int>(p.off.size());
+  t.key = ar.take<int2>(std::max<size_t>(p.key.size(), 1));
+  t.ent = ar.take<int>(std::max<size_t>(p.ent.size(), 1));
+  return t;
+}
+
+cudaError_t upload_tables(cudaStream_t st, char* ws, const Plan& p, const Tables& t,
+                          const CellTags& tags, Run& run) {
+  int* off = reinterpret_cast<int*>(ws + t.off);
+  int2* key = reinterpret_cast<int2*>(ws + t.key);
+  int* ent = reinterpret_cast<int*>(ws + t.ent);
+  run.g = p.g;
+  run.E = Entries{off, key, ent, tags};
+  run.ll = reinterpret_cast<uint64_t*>(ws + t.ll);
+  cudaError_t e = cudaMemcpyAsync(off, p.off.data(), sizeof(int) * p.off.size(),
+                                  cudaMemcpyHostToDevice, st);
+  if (e == cudaSuccess && !p.key.empty())
+    e = cudaMemcpyAsync(key, p.key.data(), sizeof(int2) * p.key.size(), cudaMemcpyHostToDevice, st);
+  if (e == cudaSuccess && !p.ent.empty())
+    e = cudaMemcpyAsync(ent, p.ent.data(), sizeof(int) * p.ent.size(), cudaMemcpyHostToDevice, st);
+  if (e == cudaSuccess) e = cudaMemsetAsync(run.ll, 0, sizeof(uint64_t) * t.ll_words, st);
+  return e;
+}
+
+int sm_count(int device) {
+  int n = 0;
+  if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) {
+    cudaGetLastError();
+    return 0;
+  }
+  return n;
+}
+
 }  // namespace res
 }  // namespace fomo

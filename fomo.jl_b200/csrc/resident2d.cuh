@@ -606,6 +606,20 @@ inline int smem_extra(int wstride, int nbc_sponge) { return std::max(3 * wstride
 // Distributes the cells of the run's tags over the tiles' threads.
 void plan_entries(Plan& p, int ns, const CellTagHost& tags);
 
+// A run's tables in the context workspace: taken from the arena, then uploaded on st
+// with the exchange buffer cleared, which completes the device pointers of `run`.
+struct Tables {
+  size_t off = 0, key = 0, ent = 0, ll = 0, ll_words = 0;
+};
+Tables take_tables(Arena& ar, const Plan& p);
+cudaError_t upload_tables(cudaStream_t st, char* ws, const Plan& p, const Tables& t,
+                          const CellTags& tags, Run& run);
+// Runs of more steps than this keep their state on the chip when it fits: at every
+// size measured that halves the step.  Shorter runs gain under 2 ms a call and keep the
+// replayed launches, whose count callers read in the stats and the tests pin.
+constexpr int kMinSteps = 300;
+int sm_count(int device);
+
 // Device planes of a launch: materials and the state read (null: zero) and written.
 struct Fields {
   // acoustic bx, bz, kappa; elastic bx, bz, lam, l2m, mut; scalar c2; coupled the

@@ -263,21 +263,6 @@ int tune_sweep(fomo_ctx* ctx, cudaStream_t st, SweepPlan& sp, int N, const Geo2&
   return FOMO_OK;
 }
 
-// Runs of more steps than this keep their state on the chip when it fits: at every
-// size measured that halves the step (figures in resident2d.cuh).  Shorter runs gain
-// under 2 ms a call and keep the replayed launches, whose count callers read in the
-// stats and the tests pin.
-constexpr int kResMinSteps = 300;
-
-int sm_count(int device) {
-  int n = 0;
-  if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) {
-    cudaGetLastError();
-    return 0;
-  }
-  return n;
-}
-
 struct Outs {
   float* seis[3];
   int nseis;
@@ -392,16 +377,16 @@ int run2d(fomo_ctx* ctx, Plan2& P, const float* vp, const float* vs, const float
   // per SM).
   //
   // Runs whose state fits on the chip keep it there for the whole time loop
-  // (resident2d.cuh): AUTO's pick for more than kResMinSteps steps.
+  // (resident2d.cuh): AUTO's pick for more than res::kMinSteps steps.
   const bool prof_req = opts && (opts->flags & FOMO_F_PROFILE);
   res::Plan rp;
-  if (P.kernel == FOMO_KERNEL_AUTO && kernel == FOMO_KERNEL_TWO_PHASE && !P.fp16 && !hook && !prof_req && P.nt > kResMinSteps &&
+  if (P.kernel == FOMO_KERNEL_AUTO && kernel == FOMO_KERNEL_TWO_PHASE && !P.fp16 && !hook && !prof_req && P.nt > res::kMinSteps &&
       !(opts && (opts->flags & FOMO_F_STEP_LAUNCH)))
     rp = res::make_plan(P.phys == kAcoustic  ? res::kAcousticNeeds
                         : P.phys == kElastic ? res::kElasticNeeds
                                              : res::kScalarNeeds,
                         P.N, P.nxp,
-                        P.nzp, P.ld, hh.nbc, P.ns, sm_count(ctx->device),
+                        P.nzp, P.ld, hh.nbc, P.ns, res::sm_count(ctx->device),
                         res::smem_extra(hh.wstride, P.sponge ? P.nbc : 0));
   const bool tagged = !rp.ok && !P.fp16 && !hook && (long long)P.nxp * P.nzp * P.ns <= 2000000LL &&
                       (P.phys == kScalar || kernel == FOMO_KERNEL_TWO_PHASE);
@@ -415,11 +400,7 @@ int run2d(fomo_ctx* ctx, Plan2& P, const float* vp, const float* vs, const float
   size_t o_list =
       tagged || rp.ok ? ar.take<int32_t>(std::max<size_t>(tags.list.size(), 1)) : 0;
   if (rp.ok) res::plan_entries(rp, P.ns, tags);
-  const size_t ll_words = rp.ok ? (size_t)4 * rp.tiles * rp.g.per : 0;
-  size_t o_ll = rp.ok ? ar.take<uint64_t>(ll_words) : 0;
-  size_t o_roff = rp.ok ? ar.take<int>(rp.off.size()) : 0;
-  size_t o_rkey = rp.ok ? ar.take<int2>(std::max<size_t>(rp.key.size(), 1)) : 0;
-  size_t o_rent = rp.ok ? ar.take<int>(std::max<size_t>(rp.ent.size(), 1)) : 0;
+  const res::Tables rt = res::take_tables(ar, rp);
   size_t o_pack = sweep ? ar.take<float>(sweep_pack_floats(P.nxp, P.nzp)) : 0;
   size_t o_ppack = pair_ok ? ar.take<float>(pair_pack_floats(P.nxp, P.nzp)) : 0;
   // replica: strip backups of the five fields, three weight planes, frame scratch
@@ -718,24 +699,12 @@ int run2d(fomo_ctx* ctx, Plan2& P, const float* vp, const float* vs, const float
   };
   // ---- the time loop on the chip ----
   if (rp.ok) {
-    FOMO_CU(ctx, cudaMemcpyAsync(ws_ptr<int>(ctx, o_roff), rp.off.data(),
-                                 sizeof(int) * rp.off.size(), cudaMemcpyHostToDevice, st));
-    if (!rp.key.empty()) {
-      FOMO_CU(ctx, cudaMemcpyAsync(ws_ptr<int2>(ctx, o_rkey), rp.key.data(),
-                                   sizeof(int2) * rp.key.size(), cudaMemcpyHostToDevice, st));
-      FOMO_CU(ctx, cudaMemcpyAsync(ws_ptr<int>(ctx, o_rent), rp.ent.data(),
-                                   sizeof(int) * rp.ent.size(), cudaMemcpyHostToDevice, st));
-    }
     res::Run run;
-    run.g = rp.g;
     run.c = c;
     run.dtx = dtx;
     run.dtz = dtz;
     run.h = h;
-    run.E = res::Entries{ws_ptr<int>(ctx, o_roff), ws_ptr<int2>(ctx, o_rkey),
-                         ws_ptr<int>(ctx, o_rent), tg};
-    run.ll = ws_ptr<uint64_t>(ctx, o_ll);
-    FOMO_CU(ctx, cudaMemsetAsync(run.ll, 0, sizeof(uint64_t) * ll_words, st));
+    FOMO_CU(ctx, res::upload_tables(st, static_cast<char*>(ctx->ws), rp, rt, tg, run));
     run.snap_interval = d_snap ? P.snap_interval : 0;
     run.pad = P.pad;
     run.nxi = P.nx;

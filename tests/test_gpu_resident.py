@@ -124,6 +124,20 @@ def test_scalar2d_on_chip(fomo, both, nx, nz, nbc, order):
     assert np.abs(a[0].seis_u).max() > 0
 
 
+@pytest.mark.parametrize("nx,nz,nbc", SIZES[:-1] + [(410, 310, 15)])
+@pytest.mark.parametrize("order", [2, 4, 6, 8, 10])
+def test_coupled2d_on_chip(fomo, both, nx, nz, nbc, order):
+    vp, _ = _layers(nx, nz, nx + order)
+    vp = np.minimum(vp, np.float32(3000.0))
+    vs = np.asfortranarray((vp / 1.8).astype(np.float32))
+    rx = np.arange(1, nx + 1, 3)
+    kw = dict(sx=[nx // 2 + 1, 1, nx], sz=[nz // 2 + 1, 1, nz], rx=rx,
+              rz=np.full(rx.size, min(3, nz)), nbc=nbc, fd_order=order, snap_interval=35)
+    a, b = both(fomo.coupled2d, vp, vs, 10.0, 1e-3, NT, 15.0, **kw)
+    _same(a[0], b[0])
+    assert np.abs(a[0].seis_P).max() > 0
+
+
 @pytest.mark.parametrize("order", [2, 8, 10])
 def test_acoustic2d_sponge_on_chip(fomo, both, order):
     vp, rho = _layers(150, 111, 4)
