@@ -30,7 +30,7 @@ Plan make_plan(const Needs& nd, int N, int nx, int nz, int ld, int nbc, int ns, 
     const int gz = std::max(1, std::min(per / gx, nz / H));
     for (int z = std::max(1, gz - 2); z <= gz; ++z) {
       const int TH = (nz + z - 1) / z;
-      for (int form = 0; form < kNumForms; ++form) {
+      for (int form = 0; form < nd.forms; ++form) {
         const int R = kForms[form].R, CX = kForms[form].CX, nb = 4 * nq / CX;
         const int ngr = (TH + 2 + R - 1) / R, thr = nb * ngr;
         if (thr > kForms[form].threads) continue;
@@ -38,30 +38,33 @@ Plan make_plan(const Needs& nd, int N, int nx, int nz, int ld, int nbc, int ns, 
         // columns: L + the quads + the right halo, padded so that the 16-byte reads
         // of a warp that spans row groups miss each other's banks
         const int need = L + 4 * nq + (N == 5 ? 8 : 4);
-        for (int pad = 28; pad >= 0; pad -= 4) {
-          const int pitch = need + pad;
-          if (pad && (R * (pitch / 4) - nq) % 8 != 0) continue;
-          const int floats = (nd.hal * rows * pitch +
-                              (nd.ext + (CX * R > nd.mreg ? nd.mats : 0)) * ngr * R * 4 * nq + extra + 3) &
-                             ~3;
-          // words put (4 bytes of table each) and got (8 bytes) by both half steps
-          const int put = (2 * N + 1 + nd.wide) * (nd.strips * TH + nd.bands * TW) +
-                          2 * (nd.rows * TW + nd.cols * TH);
-          const int get = put + 2 * (2 * N + 1 + nd.wide) * (nd.strips + nd.bands);
-          const size_t smem = sizeof(float) * floats + sizeof(int) * (put + 2) + sizeof(Word) * get;
-          if (smem > (size_t)kMaxSmem) continue;
-          // the slowest tile sets the pace: its extended cells, plus the halo it reads
-          const double cost = 4.0 * R * nq * ngr + form + 2.0 * (TW + TH) * (2 * N + 2) * 0.3;
-          if (best.ok && cost >= best_cost) continue;
-          best_cost = cost;
-          best.ok = true;
-          best.form = form;
-          // idle threads of a small tile still move words
-          best.threads = (std::min(kForms[form].threads, std::max(thr, get / 6)) + 31) & ~31;
-          best.tiles = gx * z * ns;
-          best.smem = smem;
-          best.g = Geom{nx, nz, ld, (long long)ld * nz, N, nbc, gx, z, nq, ngr, nb, pitch, rows, floats, put};
-        }
+        const bool mreg = CX * R <= nd.mreg, small = CX * R <= kSmallBlock;
+        for (int gmat = 0; gmat <= (mreg || small ? 0 : 1); ++gmat)
+          for (int pad = 28; pad >= 0; pad -= 4) {
+            const int pitch = need + pad;
+            if (pad && (R * (pitch / 4) - nq) % 8 != 0) continue;
+            const int ext = nd.ext + (mreg || gmat ? 0 : nd.mats);
+            const int floats = (nd.hal * rows * pitch + ext * ngr * R * 4 * nq + extra + 3) & ~3;
+            // words put (4 bytes of table each) and got (8 bytes) by both half steps
+            const int put = (2 * N + 1 + nd.wide) * (nd.strips * TH + nd.bands * TW) +
+                            2 * (nd.rows * TW + nd.cols * TH);
+            const int get = put + 2 * (2 * N + 1 + nd.wide) * (nd.strips + nd.bands);
+            const size_t smem = sizeof(float) * floats + sizeof(int) * (put + 2) + sizeof(Word) * get;
+            if (smem > (size_t)kMaxSmem) continue;
+            // the slowest tile sets the pace: its extended cells, plus the halo it reads
+            const double cost = 4.0 * R * nq * ngr + form + 2.0 * (TW + TH) * (2 * N + 2) * 0.3 +
+                                gmat * 1000.0;
+            if (best.ok && cost >= best_cost) continue;
+            best_cost = cost;
+            best.ok = true;
+            best.form = form;
+            // idle threads of a small tile still move words
+            best.threads = (std::min(kForms[form].threads, std::max(thr, get / 6)) + 31) & ~31;
+            best.tiles = gx * z * ns;
+            best.smem = smem;
+            best.g = Geom{nx,  nz, ld,    (long long)ld * nz, N,      nbc, gx,  z,
+                          nq, ngr, nb, pitch, rows, floats, put, gmat};
+          }
       }
     }
   }

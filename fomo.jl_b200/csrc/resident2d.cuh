@@ -20,8 +20,8 @@
 //
 // What it measured (us per step, order 8, this form / replayed two-phase launches):
 // acoustic 240x200 nbc 50 4.7 / 9.1, 400x300 nbc 100 5.9 / 12.8, 4 shots of 240x200
-// 7.4 / 14.9; elastic 240x200 6.7 / 10.5, 501x397 10.9 / 17.0; scalar 240x200 2.1 / 4.1,
-// 500x400 2.8 / 5.6.  An exchange costs about 0.7 us, the rest is issue and latency of the
+// 7.4 / 14.9, eight 13.2 / 22.9, 1000x800 12.9 / 21.7 (materials from L2); elastic 240x200 6.7 / 10.5, 501x397 10.9 / 17.0; scalar 240x200 2.1 / 4.1,
+// 500x400 2.8 / 5.6, 1000x800 5.3 / 10.5; coupled 400x300 nbc 100 9.7 / 15.0.  An exchange costs about 0.7 us, the rest is issue and latency of the
 // phases between barriers (36 % issue active at 20 warps per SM).
 //
 // A tile computes its own cells and a one-cell ring around them (the inward
@@ -48,8 +48,9 @@ namespace res {
 struct Form {
   int CX, R, threads;
 };
-constexpr Form kForms[] = {{1, 1, 1024}, {4, 1, 640}, {4, 2, 512}, {4, 4, 384}};
+constexpr Form kForms[] = {{1, 1, 1024}, {4, 1, 640}, {4, 2, 512}, {4, 4, 512}};
 constexpr int kNumForms = 4;
+constexpr int kSmallBlock = 4;  // cells of blocks that always have their materials on the chip
 
 // Decomposition and shared-memory geometry of one run (the same for every tile;
 // tiles differ by at most one column or row).
@@ -63,6 +64,7 @@ struct Geom {
   int pitch, rows;     // haloed arrays (floats per row, rows)
   int words;           // start of the word tables in shared memory (floats)
   int per;             // words a tile publishes per half step, at most
+  int gmat;            // materials are read from global memory (they do not fit on the chip)
 };
 
 // First column / row of tile i of `parts`.  Tiles start one column past a multiple
@@ -363,6 +365,25 @@ struct Work {
   __device__ __forceinline__ void load_ext(const Run& run, float* A, const float* src) const {
     load_tile(run.g, t, src, A, ep, run.g.ngr * R, t.off, 1);
   }
+  // Row k of the block in a material plane, from its extended array or, where the
+  // materials stay off the chip, from L2 (a row outside the grid reads the nearest one: its
+  // cells take no update).
+  __device__ __forceinline__ Vec<CX> mat(const Run& run, const float* A, const float* plane,
+                                         int k) const {
+    if (CX * R <= kSmallBlock || !run.g.gmat) return ldv<CX>(A + eb + k * ep);
+    const float* p = plane + (long long)min(max(cl.z + k, 0), run.g.nz - 1) * run.g.ld + cl.x;
+    Vec<CX> r;
+    if constexpr (CX == 4) {
+      const float4 q = __ldg(reinterpret_cast<const float4*>(p));
+      r.v[0] = q.x;
+      r.v[1] = q.y;
+      r.v[2] = q.z;
+      r.v[3] = q.w;
+    } else {
+      r.v[0] = cl.x < run.g.nx ? __ldg(p) : 0.0f;
+    }
+    return r;
+  }
   // the block's cells of a material plane (zero outside the grid)
   __device__ __forceinline__ void load_own(const Run& run, float (&m)[R][CX], const float* src) const {
 #pragma unroll
@@ -587,16 +608,18 @@ struct Plan {
 };
 
 // What a solver keeps in shared memory: `hal` haloed arrays, `ext` arrays over the
-// extended tile, `mats` materials (extended arrays too where blocks have over
-// mreg cells, else in registers) and the words of its regions (counts per kind).
+// extended tile, `mats` materials (in registers where blocks have up to mreg cells,
+// else extended arrays, or off the chip where those do not fit) and the words of its regions (counts per kind).
 struct Needs {
   int hal, ext, mats, mreg, strips, bands, rows, cols;
   int wide;  // strips and bands are 2N + 1 + wide cells wide in all
+  int forms; // block forms in use: 4 x 4 blocks of the elastic and coupled updates spill
+             // (elastic 700x600 30.2 us per step against 23.2 launched)
 };
-constexpr Needs kAcousticNeeds{3, 2, 3, 8, 2, 2, 1, 1, 0};
-constexpr Needs kElasticNeeds{5, 3, 5, 0, 4, 4, 1, 1, 0};
-constexpr Needs kScalarNeeds{1, 1, 1, 8, 1, 1, 0, 0, 1};
-constexpr Needs kCoupledNeeds{4, 2, 8, 0, 2, 2, 2, 2, 1};
+constexpr Needs kAcousticNeeds{3, 2, 3, 8, 2, 2, 1, 1, 0, 4};
+constexpr Needs kElasticNeeds{5, 3, 5, 0, 4, 4, 1, 1, 0, 3};
+constexpr Needs kScalarNeeds{1, 1, 1, 8, 1, 1, 0, 0, 1, 4};
+constexpr Needs kCoupledNeeds{4, 2, 8, 0, 2, 2, 2, 2, 1, 3};
 // Chooses the tiles of a run (extra: floats of the weight ramps); ok = false when it
 // does not fit on the chip.
 Plan make_plan(const Needs& needs, int N, int nx, int nz, int ld, int nbc, int ns, int nsm,
@@ -648,7 +671,8 @@ cudaError_t launch_elastic(cudaStream_t st, int N, bool sponge, const Plan& p, c
                            const Fields& f);
 
 // switch over the block forms: M(index, CX, R, threads)
-#define FOMO_RES_FORMS(M) M(0, 1, 1, 1024) M(1, 4, 1, 640) M(2, 4, 2, 512) M(3, 4, 4, 384)
+#define FOMO_RES_FORMS3(M) M(0, 1, 1, 1024) M(1, 4, 1, 640) M(2, 4, 2, 512)
+#define FOMO_RES_FORMS(M) FOMO_RES_FORMS3(M) M(3, 4, 4, 512)
 
 template <class Kern, class... More>
 cudaError_t launch_resident(cudaStream_t st, Kern kern, const Plan& p, const Run& run,

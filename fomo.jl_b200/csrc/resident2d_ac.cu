@@ -27,7 +27,7 @@ __global__ void __launch_bounds__(THREADS, 1)
   float* U0 = P + hn;
   float* U1 = U0 + en;
   float* ME = U1 + en;
-  float* wt = ME + (MREG ? 0 : 3 * en);
+  float* wt = ME + (MREG || g.gmat ? 0 : 3 * en);
   const long long so = (long long)w.t.shot * g.plane;
   w.load(run, P, f.in[2] ? f.in[2] + so : nullptr);
   w.load(run, VX, f.in[0] ? f.in[0] + so : nullptr);
@@ -43,7 +43,7 @@ __global__ void __launch_bounds__(THREADS, 1)
         mr[0][k][j] = __fmul_rn(mr[0][k][j], run.dtx);
         mr[1][k][j] = __fmul_rn(mr[1][k][j], run.dtz);
       }
-  } else {
+  } else if (!g.gmat) {
     for (int i = 0; i < 3; ++i) w.load_ext(run, ME + i * en, f.mat[i]);
     __syncthreads();
     for (int i = threadIdx.x; i < en; i += blockDim.x) {
@@ -57,7 +57,14 @@ __global__ void __launch_bounds__(THREADS, 1)
 #pragma unroll
       for (int j = 0; j < CX; ++j) v.v[j] = mr[i][k][j];
       return v;
-    } else return ldv<CX>(ME + i * en + w.eb + k * w.ep);
+    } else {
+      Vec<CX> v = w.mat(run, ME + i * en, f.mat[i], k);
+      if (i < 2 && g.gmat) {
+#pragma unroll
+        for (int j = 0; j < CX; ++j) v.v[j] = __fmul_rn(v.v[j], i ? run.dtz : run.dtx);
+      }
+      return v;
+    }
   };
   const int nwt = SP ? run.h.nbc : 3 * run.h.wstride;
   for (int i = threadIdx.x; i < nwt; i += blockDim.x) wt[i] = __ldg(run.h.wtab + i);

@@ -62,9 +62,10 @@ __global__ void __launch_bounds__(THREADS, 1)
   float* U0 = DS + hn;
   float* U1 = U0 + en;
   float* ME = U1 + en;  // alpha, beta, their x and z derivatives, Laplacians
-  float* wt = ME + 8 * en;
+  float* wt = ME + (g.gmat ? 0 : 8 * en);
   for (int i = 0; i < 4; ++i) w.load(run, P + i * hn, f.in[i]);
-  for (int i = 0; i < 8; ++i) w.load_ext(run, ME + i * en, f.mat[i]);
+  if (!g.gmat)
+    for (int i = 0; i < 8; ++i) w.load_ext(run, ME + i * en, f.mat[i]);
   for (int i = threadIdx.x; i < 3 * run.h.wstride; i += blockDim.x) wt[i] = __ldg(run.h.wtab + i);
   // halo regions: dP/dt and dS/dt in the ring, P and S along x and z
   const Region rv[4] = {{kRows, 0, 0, 2}, {kCols, 0, 0, 2}, {kRows, 0, 0, 3}, {kCols, 0, 0, 3}};
@@ -82,7 +83,7 @@ __global__ void __launch_bounds__(THREADS, 1)
   for (int step = 0; step < run.nsteps; ++step) {
     const int it = run.it0 + step;
     w.refresh();
-    const int hb = w.hb, eb = w.eb, pitch = w.pitch, ep = w.ep;
+    const int hb = w.hb, pitch = w.pitch;
     uint64_t* l0 = run.ll + (long long)(it & 1) * 2 * gridDim.x * g.per;
     uint64_t* l1 = l0 + (long long)gridDim.x * g.per;
     const long long part = (long long)blockIdx.x * g.per;
@@ -95,12 +96,10 @@ __global__ void __launch_bounds__(THREADS, 1)
       s.load(S, hb, pitch, c);
 #pragma unroll
       for (int k = 0; k < R; ++k) {
-        const int e = eb + k * ep;
         const Vec<CX> oP = ldv<CX>(DP + hb + k * pitch), oS = ldv<CX>(DS + hb + k * pitch);
-        const Vec<CX> a = ldv<CX>(ME + e), b = ldv<CX>(ME + en + e), ax = ldv<CX>(ME + 2 * en + e),
-                      az = ldv<CX>(ME + 3 * en + e), bx = ldv<CX>(ME + 4 * en + e),
-                      bz = ldv<CX>(ME + 5 * en + e), la = ldv<CX>(ME + 6 * en + e),
-                      lb = ldv<CX>(ME + 7 * en + e);
+        auto med = [&](int i) { return w.mat(run, ME + i * en, f.mat[i], k); };
+        const Vec<CX> a = med(0), b = med(1), ax = med(2), az = med(3), bx = med(4), bz = med(5),
+                      la = med(6), lb = med(7);
 #pragma unroll
         for (int j = 0; j < CX; ++j) {
           const float Pc = p.mid[k][j];
@@ -183,7 +182,7 @@ cudaError_t launch_coupled(cudaStream_t st, int N, const Plan& p, const Run& run
   case I: return launch_resident(st, k_res_cp<NN, CX, R, T>, p, run, f, c);
   auto go = [&](auto n) -> cudaError_t {
     constexpr int NN = decltype(n)::value;
-    switch (p.form) { FOMO_RES_FORMS(FOMO_RES_F) }
+    switch (p.form) { FOMO_RES_FORMS3(FOMO_RES_F) }
     return cudaErrorInvalidValue;
   };
 #undef FOMO_RES_F

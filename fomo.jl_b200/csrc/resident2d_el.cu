@@ -26,16 +26,13 @@ __global__ void __launch_bounds__(THREADS, 1)
   float* ZZ = XX + hn;
   float* XZ = ZZ + hn;
   float* M = XZ + hn;  // bx, bz, lam, l2m, mut
-  float* U = M + 5 * en;
+  float* U = M + (g.gmat ? 0 : 5 * en);
   float* wt = U + 3 * en;
   const long long so = (long long)w.t.shot * g.plane;
 #pragma unroll
   for (int i = 0; i < 5; ++i) w.load(run, VX + i * hn, f.in[i] ? f.in[i] + so : nullptr);
-  w.load_ext(run, M, f.mat[0]);
-  w.load_ext(run, M + en, f.mat[1]);
-  w.load_ext(run, M + 2 * en, f.mat[2]);
-  w.load_ext(run, M + 3 * en, f.mat[3]);
-  w.load_ext(run, M + 4 * en, f.mat[4]);
+  if (!g.gmat)
+    for (int i = 0; i < 5; ++i) w.load_ext(run, M + i * en, f.mat[i]);
   const int nwt = SP ? run.h.nbc : 3 * run.h.wstride;
   for (int i = threadIdx.x; i < nwt; i += blockDim.x) wt[i] = __ldg(run.h.wtab + i);
   // halo regions: vx, vz and txz are read along x and z, txx along x and tzz along z (and
@@ -56,7 +53,7 @@ __global__ void __launch_bounds__(THREADS, 1)
   for (int step = 0; step < run.nsteps; ++step) {
     const int it = run.it0 + step;
     w.refresh();
-    const int hb = w.hb, eb = w.eb, pitch = w.pitch, ep = w.ep;
+    const int hb = w.hb, pitch = w.pitch;
     // this step's buffers of the two half steps, and this tile's parts
     uint64_t* l0 = run.ll + (long long)(it & 1) * 2 * gridDim.x * g.per;
     uint64_t* l1 = l0 + (long long)gridDim.x * g.per;
@@ -85,9 +82,9 @@ __global__ void __launch_bounds__(THREADS, 1)
 #pragma unroll
         for (int k = 0; k < R; ++k) {
           XWin<N, CX> xw;
-          const int h = hb + k * pitch, e = eb + k * ep;
+          const int h = hb + k * pitch;
           xw.load(XX + h);
-          const Vec<CX> ox = ldv<CX>(VX + h), bx = ldv<CX>(M + e);
+          const Vec<CX> ox = ldv<CX>(VX + h), bx = w.mat(run, M, f.mat[0], k);
 #pragma unroll
           for (int j = 0; j < CX; ++j) {
             const float u = __fmaf_rn(bx[j], __fmaf_rn(run.dtx, xw.dm(j, c), ux[k][j]),
@@ -96,7 +93,7 @@ __global__ void __launch_bounds__(THREADS, 1)
             if constexpr (SP) ux[k][j] = w.damp(run, wt, k, j, ux[k][j]);
           }
           xw.load(XZ + h);
-          const Vec<CX> oz = ldv<CX>(VZ + h), bz = ldv<CX>(M + en + e);
+          const Vec<CX> oz = ldv<CX>(VZ + h), bz = w.mat(run, M + en, f.mat[1], k);
 #pragma unroll
           for (int j = 0; j < CX; ++j) {
             const float u = __fmaf_rn(bz[j], __fmaf_rn(run.dtx, xw.dp(j, c), uz[k][j]),
@@ -139,10 +136,10 @@ __global__ void __launch_bounds__(THREADS, 1)
 #pragma unroll
       for (int k = 0; k < R; ++k) {
         XWin<N, CX> xw;
-        const int h = hb + k * pitch, e = eb + k * ep;
+        const int h = hb + k * pitch;
         xw.load(VX + h);
         const Vec<CX> oxx = ldv<CX>(XX + h), ozz = ldv<CX>(ZZ + h);
-        const Vec<CX> la = ldv<CX>(M + 2 * en + e), l2 = ldv<CX>(M + 3 * en + e);
+        const Vec<CX> la = w.mat(run, M + 2 * en, f.mat[2], k), l2 = w.mat(run, M + 3 * en, f.mat[3], k);
 #pragma unroll
         for (int j = 0; j < CX; ++j) {
           const float ex = __fmul_rn(xw.dp(j, c), run.dtx), ez = sz[k][j];
@@ -158,7 +155,7 @@ __global__ void __launch_bounds__(THREADS, 1)
           }
         }
         xw.load(VZ + h);
-        const Vec<CX> oxz = ldv<CX>(XZ + h), mu = ldv<CX>(M + 4 * en + e);
+        const Vec<CX> oxz = ldv<CX>(XZ + h), mu = w.mat(run, M + 4 * en, f.mat[4], k);
 #pragma unroll
         for (int j = 0; j < CX; ++j) {
           const float u = __fmaf_rn(mu[j],
@@ -224,7 +221,7 @@ cudaError_t launch_elastic(cudaStream_t st, int N, bool sponge, const Plan& p, c
                   : launch_resident(st, k_res_el<NN, CX, R, T, false>, p, run, f);
   auto go = [&](auto n) -> cudaError_t {
     constexpr int NN = decltype(n)::value;
-    switch (p.form) { FOMO_RES_FORMS(FOMO_RES_F) }
+    switch (p.form) { FOMO_RES_FORMS3(FOMO_RES_F) }
     return cudaErrorInvalidValue;
   };
 #undef FOMO_RES_F

@@ -25,11 +25,11 @@ __global__ void __launch_bounds__(THREADS, 1)
   float* A = sm;
   float* U = A + hn;
   float* ME = U + en;
-  float* wt = ME + (MREG ? 0 : en);
+  float* wt = ME + (MREG || g.gmat ? 0 : en);
   w.load(run, A, f.in[0]);
   float mr[R][CX], u0[R][CX];
   if constexpr (MREG) w.load_own(run, mr, f.mat[0]);
-  else w.load_ext(run, ME, f.mat[0]);
+  else if (!g.gmat) w.load_ext(run, ME, f.mat[0]);
 #pragma unroll
   for (int k = 0; k < R; ++k)
 #pragma unroll
@@ -57,6 +57,8 @@ __global__ void __launch_bounds__(THREADS, 1)
       for (int k = 0; k < R; ++k) {
         XWin<N, CX> xw;
         xw.load(A + hb + k * pitch);
+        Vec<CX> c2;
+        if constexpr (!MREG) c2 = w.mat(run, ME, f.mat[0], k);
 #pragma unroll
         for (int j = 0; j < CX; ++j) {
           constexpr int L = XWin<N, CX>::L;
@@ -69,8 +71,7 @@ __global__ void __launch_bounds__(THREADS, 1)
                                        zw[N + k - l][j]);
             lap = __fmaf_rn(c.d2[l - 1], nb, lap);
           }
-          const float c2 = MREG ? mr[k][j] : ME[w.eb + k * w.ep + j];
-          const float v = __fmaf_rn(c2, lap, __fsub_rn(__fmul_rn(2.0f, uc), u0[k][j]));
+          const float v = __fmaf_rn(MREG ? mr[k][j] : c2[j], lap, __fsub_rn(__fmul_rn(2.0f, uc), u0[k][j]));
           u[k][j] = w.inner(k, j) ? v : uc;
           u0[k][j] = uc;
         }

@@ -56,8 +56,10 @@ def _layers(nx, nz, seed):
 
 
 # one tile's width and height, ragged tiles, a grid too flat or too narrow for
-# many tiles, no absorbing layer beyond the stencil, larger blocks per thread
-SIZES = [(33, 29, 10), (171, 90, 12), (401, 7, 3), (5, 260, 6), (120, 100, 1), (640, 470, 20)]
+# many tiles, no absorbing layer beyond the stencil, larger blocks per thread,
+# materials off the chip
+SIZES = [(33, 29, 10), (171, 90, 12), (401, 7, 3), (5, 260, 6), (120, 100, 1), (640, 470, 20),
+         (910, 760, 20)]
 
 
 @pytest.mark.parametrize("nx,nz,nbc", SIZES)
@@ -78,7 +80,7 @@ def test_acoustic2d_on_chip(fomo, both, nx, nz, nbc, order):
     assert np.abs(a[0].seis_p).max() > 0
 
 
-@pytest.mark.parametrize("nx,nz,nbc", SIZES[:-1] + [(430, 330, 20)])
+@pytest.mark.parametrize("nx,nz,nbc", SIZES[:-2] + [(430, 330, 20), (620, 540, 9)])
 @pytest.mark.parametrize("order", [2, 4, 6, 8, 10])
 def test_elastic2d_on_chip(fomo, both, nx, nz, nbc, order):
     vp, rho = _layers(nx, nz, nx + order)
@@ -124,7 +126,7 @@ def test_scalar2d_on_chip(fomo, both, nx, nz, nbc, order):
     assert np.abs(a[0].seis_u).max() > 0
 
 
-@pytest.mark.parametrize("nx,nz,nbc", SIZES[:-1] + [(410, 310, 15)])
+@pytest.mark.parametrize("nx,nz,nbc", SIZES[:-2] + [(410, 310, 15), (590, 560, 9)])
 @pytest.mark.parametrize("order", [2, 4, 6, 8, 10])
 def test_coupled2d_on_chip(fomo, both, nx, nz, nbc, order):
     vp, _ = _layers(nx, nz, nx + order)
