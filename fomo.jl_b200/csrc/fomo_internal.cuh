@@ -23,6 +23,10 @@ struct fomo_ctx {
   void* ws = nullptr;  // device workspace, grown on demand and reused
   size_t ws_bytes = 0;
   int* d_flag = nullptr;  // device status word (non-finite sentinel)
+  // pinned staging of large model uploads (upload() in api.cu): kPinSlots chunks, each with
+  // the event of the copy that last read it; made on first use, freed by fomo_trim
+  char* pin = nullptr;
+  cudaEvent_t pin_ev[8] = {};
   std::string err;
 };
 
@@ -49,6 +53,8 @@ struct Arena {
   }
 };
 int ensure_workspace(fomo_ctx* ctx, size_t bytes);
+// Host to device on st; src may be reused when it returns.
+cudaError_t upload(fomo_ctx* ctx, void* dst, const void* src, size_t bytes, cudaStream_t st);
 template <class T>
 inline T* ws_ptr(fomo_ctx* ctx, size_t off) {
   return reinterpret_cast<T*>(static_cast<char*>(ctx->ws) + off);

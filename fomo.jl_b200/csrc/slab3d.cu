@@ -231,10 +231,10 @@ int fomo_slab3d_create(fomo_ctx* ctx, int32_t elastic, const fomo_grid3d* gp, co
   auto cu = [&](cudaError_t e, const char* where) {
     if (e != cudaSuccess && rc == FOMO_OK) rc = cuda_fail(ctx, e, where);
   };
-  cu(cudaMemcpyAsync(raw, vp + off, 4 * nraw, cudaMemcpyHostToDevice, st), "slab vp");
-  cu(cudaMemcpyAsync(raw + 2 * nraw, rho + off, 4 * nraw, cudaMemcpyHostToDevice, st), "slab rho");
+  cu(upload(ctx, raw, vp + off, 4 * nraw, st), "slab vp");
+  cu(upload(ctx, raw + 2 * nraw, rho + off, 4 * nraw, st), "slab rho");
   if (elastic)
-    cu(cudaMemcpyAsync(raw + nraw, vs + off, 4 * nraw, cudaMemcpyHostToDevice, st), "slab vs");
+    cu(upload(ctx, raw + nraw, vs + off, 4 * nraw, st), "slab vs");
   cu(cudaMemcpyAsync(s->wt, wt3.data(), 4 * wt3.size(), cudaMemcpyHostToDevice, st), "slab ramps");
   cu(cudaMemcpyAsync(s->src, src_lin.data(), 4 * src_lin.size(), cudaMemcpyHostToDevice, st),
      "slab sources");

@@ -416,15 +416,14 @@ int run2d(fomo_ctx* ctx, Plan2& P, const float* vp, const float* vs, const float
   const float* d_wav = acq->wavelet;
   if (!P.dev) {
     float* m = ws_ptr<float>(ctx, o_model);
-    FOMO_CU(ctx, cudaMemcpyAsync(m, vp, sizeof(float) * nint, cudaMemcpyHostToDevice, st));
+    FOMO_CU(ctx, upload(ctx, m, vp, sizeof(float) * nint, st));
     d_vp = m;
     if (vs) {
-      FOMO_CU(ctx, cudaMemcpyAsync(m + nint, vs, sizeof(float) * nint, cudaMemcpyHostToDevice, st));
+      FOMO_CU(ctx, upload(ctx, m + nint, vs, sizeof(float) * nint, st));
       d_vs = m + nint;
     }
     if (rho) {
-      FOMO_CU(ctx,
-              cudaMemcpyAsync(m + 2 * nint, rho, sizeof(float) * nint, cudaMemcpyHostToDevice, st));
+      FOMO_CU(ctx, upload(ctx, m + 2 * nint, rho, sizeof(float) * nint, st));
       d_rho = m + 2 * nint;
     }
     if (P.n_src > 0) {

@@ -823,12 +823,12 @@ int run3d(fomo_ctx* ctx, bool elastic, const fomo_grid3d* gp, const float* vp, c
   const float* d_wav = acq->wavelet;
   if (!dev) {
     float* m = ws_ptr<float>(ctx, o_model);
-    FOMO_CU(ctx, cudaMemcpyAsync(m, vp, 4 * nint, cudaMemcpyHostToDevice, st));
-    FOMO_CU(ctx, cudaMemcpyAsync(m + 2 * nint, rho, 4 * nint, cudaMemcpyHostToDevice, st));
+    FOMO_CU(ctx, upload(ctx, m, vp, 4 * nint, st));
+    FOMO_CU(ctx, upload(ctx, m + 2 * nint, rho, 4 * nint, st));
     d_vp = m;
     d_rho = m + 2 * nint;
     if (elastic) {
-      FOMO_CU(ctx, cudaMemcpyAsync(m + nint, vs, 4 * nint, cudaMemcpyHostToDevice, st));
+      FOMO_CU(ctx, upload(ctx, m + nint, vs, 4 * nint, st));
       d_vs = m + nint;
     }
     if (acq->n_src) {

@@ -772,7 +772,7 @@ int run_uneven(fomo_ctx* ctx, float dh, float dt, int nt, int nbc, int fd_order,
       wstride = hh.wstride;
       zone = hh.nbc;
     }
-    off_model = std::max(off_model, 2 * nint);
+    off_model += 2 * nint;
     cells += (long long)u.nx * u.nz;
   }
 
@@ -840,22 +840,24 @@ int run_uneven(fomo_ctx* ctx, float dh, float dt, int nt, int nbc, int fd_order,
   int* d_tiles = ws_ptr<int>(ctx, o_tiles);
   float* d_w = ws_ptr<float>(ctx, o_w);
 
-  // ---- materials per shot (device preparation, one model staging buffer) ----
+  // ---- materials per shot (device preparation; every shot has its staging place, so
+  // the shots follow each other without a wait) ----
   const float dtdh = dt / dh;
+  long long at_model = 0;
   for (int s = 0; s < ns; ++s) {
     const fomo_shot2d& in = shots[s];
     const long long nint = (long long)in.nx * in.nz;
-    FOMO_CU(ctx, cudaMemcpyAsync(d_model, in.vp, 4 * nint, cudaMemcpyHostToDevice, st));
-    FOMO_CU(ctx, cudaMemcpyAsync(d_model + nint, in.rho, 4 * nint, cudaMemcpyHostToDevice, st));
+    float* raw = d_model + at_model;
+    at_model += 2 * nint;
+    FOMO_CU(ctx, upload(ctx, raw, in.vp, 4 * nint, st));
+    FOMO_CU(ctx, upload(ctx, raw + nint, in.rho, 4 * nint, st));
     float* m = d_mat + tab[s].mat;
-    FOMO_CU(ctx, launch_medium2d(st, 1, in.nx, in.nz, pad, tab[s].ld, dtdh, d_model, nullptr,
-                                 d_model + nint, m, m + tab[s].plane, m + 2 * tab[s].plane, nullptr,
+    FOMO_CU(ctx, launch_medium2d(st, 1, in.nx, in.nz, pad, tab[s].ld, dtdh, raw, nullptr,
+                                 raw + nint, m, m + tab[s].plane, m + 2 * tab[s].plane, nullptr,
                                  nullptr));
     if (in.n_src)
       FOMO_CU(ctx, cudaMemcpyAsync(d_wav + tab[s].wav0, in.wavelet, 4LL * in.n_src * nt,
                                    cudaMemcpyHostToDevice, st));
-    // the staging buffer is reused by the next shot: wait for this one's reads
-    FOMO_CU(ctx, cudaStreamSynchronize(st));
   }
   if (!src_lin.empty())
     FOMO_CU(ctx, cudaMemcpyAsync(d_src, src_lin.data(), 4 * src_lin.size(), cudaMemcpyHostToDevice, st));

@@ -30,7 +30,7 @@ FOMO_KERNEL_AUTO, FOMO_KERNEL_TWO_PHASE, FOMO_KERNEL_SINGLE_SWEEP = 0, 1, 2
 # Every symbol include/fomo_b200.h declares (checked by the ABI tests).
 EXPORTS = (
     "fomo_version", "fomo_create", "fomo_destroy", "fomo_last_error", "fomo_set_stream",
-    "fomo_trim", "fomo_check_numerics", "fomo_acoustic2d", "fomo_acoustic2d_batch",
+    "fomo_trim", "fomo_check_numerics", "fomo_min_positive", "fomo_acoustic2d", "fomo_acoustic2d_batch",
     "fomo_elastic2d", "fomo_elastic2d_batch", "fomo_scalar2d", "fomo_debug_medium2d",
     "fomo_scalar2d_noalloc", "fomo_acoustic3d", "fomo_elastic3d", "fomo_acoustic2d_uneven",
     "fomo_corr_param_count", "fomo_corr_features", "fomo_corr_target", "fomo_corr_forward",
@@ -117,6 +117,8 @@ def lib() -> C.CDLL:
             L.fomo_trim.argtypes = [vp]
             L.fomo_check_numerics.argtypes = [f32, f32, f32, i32, i32, C.POINTER(C.c_float)]
             L.fomo_check_numerics.restype = C.c_int
+            L.fomo_min_positive.argtypes = [vp, C.c_int64]
+            L.fomo_min_positive.restype = C.c_float
             g, a, o, s = C.POINTER(Grid2D), C.POINTER(Acq), C.POINTER(Opts), C.POINTER(Stats)
             L.fomo_acoustic2d.argtypes = [vp, g, vp, vp, a, i32, vp, vp, vp, vp, o, s]
             L.fomo_acoustic2d_batch.argtypes = [vp, g, vp, vp, a, vp, vp, vp, o, s]

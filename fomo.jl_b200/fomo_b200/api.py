@@ -174,16 +174,10 @@ def _check_numerics(vmax, vmin_disp, dh, dt, f0, fd_order, centered=False):
 
 
 def _min_pos(a) -> np.float32:
-    """minimum(vp[vp .> 0]): scanned in memory order, in chunks (a boolean index
-    of a column-major volume would walk it in row-major order)."""
+    """minimum(vp[vp .> 0]): scanned in memory order by the library's host threads (numpy's
+    boolean index took 47 ms on a 48 M cell volume)."""
     flat = np.asarray(a, dtype=np.float32).ravel(order="K")
-    best = np.float32(np.inf)
-    step = 1 << 22
-    for i in range(0, flat.size, step):
-        c = flat[i:i + step]
-        c = c[c > 0]
-        if c.size:
-            best = min(best, np.float32(c.min()))
+    best = L.lib().fomo_min_positive(_ptr(flat), flat.size)
     if not np.isfinite(best):
         raise ArgumentError("model has no positive velocity")
     return np.float32(best)
@@ -515,8 +509,8 @@ def acoustic2d_uneven(vps, rhos, dh, dt, nt, f0, *, sx, sz, rx, rz, nbc: int = 5
     dh, dt, f0 = np.float32(dh), np.float32(dt), np.float32(f0)
     models = [(_f32F(v), _f32F(r)) for v, r in zip(vps, rhos)]
     vmax = max(float(v.max()) for v, _ in models)
-    vmin = min(float(_min_pos(v)) for v, _ in models)
-    _check_numerics(vmax, vmin, dh, dt, f0, fd_order)
+    vmins = [_min_pos(v) for v, _ in models]
+    _check_numerics(vmax, float(min(vmins)), dh, dt, f0, fd_order)
     w = _wavelet_row(wavelet, f0, dt, nt)
     if scale_source_by_dt:
         w = (w * dt).astype(np.float32)
@@ -535,7 +529,7 @@ def acoustic2d_uneven(vps, rhos, dh, dt, nt, f0, *, sx, sz, rx, rz, nbc: int = 5
         wm = np.asfortranarray(np.repeat(w[None, :], sxv.size, axis=0))
         seis = [np.zeros((rxv.size, nt), dtype=np.float32, order="F") for _ in range(3)]
         vr = v_ref[s] if isinstance(v_ref, (list, tuple, np.ndarray)) else v_ref
-        vr = 0.0 if vr is None else float(np.float32(vr))
+        vr = float(vmins[s]) if vr is None else float(np.float32(vr))
         d = descs[s]
         d.nx, d.nz, d.vp, d.rho = nx, nz, _ptr(vp), _ptr(rho)
         d.n_src, d.sx, d.sz, d.wavelet = sxv.size, _ptr(sxv), _ptr(szv), _ptr(wm)

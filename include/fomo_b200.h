@@ -142,6 +142,10 @@ FOMO_API int fomo_trim(fomo_ctx* ctx);
 FOMO_API int fomo_check_numerics(float vmax, float dh, float dt, int32_t fd_order, int32_t centered,
                         float* dt_max);
 
+/* Smallest positive value of n floats (host memory; NaN and values <= 0 are skipped),
+ * INFINITY if there is none: the reference's minimum(vp[vp .> 0]) (acoustic2d.jl:55). */
+FOMO_API float fomo_min_positive(const float* v, int64_t n);
+
 /* ---- solvers -------------------------------------------------------------
  * Outputs are caller-owned, sized (n_rec, nt, n_shots); `snaps` may be NULL.
  * opts may be NULL (FP32, host pointers, autotuned kernel).
