@@ -12,6 +12,7 @@
 #include <tuple>
 #include <type_traits>
 
+#include "bulk2d.cuh"
 #include "solver2d_kernels.cuh"
 #include "mixed2d.cuh"
 #include "replica2d.cuh"
@@ -262,6 +263,11 @@ int tune_sweep(fomo_ctx* ctx, cudaStream_t st, SweepPlan& sp, int N, const Geo2&
   g_tune[key] = bv;
   return FOMO_OK;
 }
+
+// Inner shot-cells from which the two-phase kernels work in blocks per thread: at 120 k
+// (acoustic 400x300) the few blocks leave SMs idle and the step takes as long either way
+// (10.8 us), at 420 k it falls from 16.8 to 12.9 us.
+constexpr long long kBulkCells = 200000;
 
 struct Outs {
   float* seis[3];
@@ -565,6 +571,12 @@ int run2d(fomo_ctx* ctx, Plan2& P, const float* vp, const float* vs, const float
   }
 
   dim3 blk(32, 8), grd(cdiv(P.nxp, 32), cdiv(P.nzp, 8), P.ns);
+  // Grids with a large inner rectangle take the block-per-thread kernels (bulk2d.cuh).
+  constexpr int kBulkR = 2;
+  const bulk::Split split = bulk::make_split(
+      g, P.sponge ? std::max(P.nbc, P.M) : hh.nbc + 1, bulk::kThreads / 32 * kBulkR);
+  const bool use_bulk = (long long)(split.x1 - split.x0) * (split.z1 - split.z0) * P.ns >= kBulkCells;
+  const dim3 bgrd(split.edge + split.tiles, 1, P.ns);
   int launches = 0;
   // FOMO_F_PROFILE: event pairs around the sweep kernel(s) of a window of steps
   const bool prof = opts && (opts->flags & FOMO_F_PROFILE) && P.nt >= 2;
@@ -633,7 +645,14 @@ int run2d(fomo_ctx* ctx, Plan2& P, const float* vp, const float* vs, const float
       switch (P.N) {
 #define FOMO_AC2_CASE(NN)                                                                        \
   case NN:                                                                                       \
-    if constexpr (TGV) {                                                                         \
+    if (use_bulk) {                                                                              \
+      bulk::k_ac_vel_bulk<NN, kBulkR, SPV><<<bgrd, bulk::kThreads, 0, s>>>(                      \
+          g, split, c, dtx, dtz, h, field(a, 2), field(a, 0), field(a, 1), bx, bz, field(b, 0),  \
+          field(b, 1));                                                                          \
+      bulk::k_ac_prs_bulk<NN, kBulkR, SPV, TGV><<<bgrd, bulk::kThreads, 0, s>>>(                 \
+          g, split, c, dtx, dtz, h, field(a, 2), field(b, 0), field(b, 1), kap, field(b, 2), tg, \
+          j);                                                                                    \
+    } else if constexpr (TGV) {                                                                  \
       k_ac_vel<NN, SPV><<<grd, blk, 0, s>>>(g, c, dtx, dtz, h, field(a, 2), field(a, 0),         \
                                             field(a, 1), bx, bz, field(b, 0), field(b, 1));      \
       k_ac_prs<NN, SPV, true><<<grd, blk, 0, s>>>(g, c, dtx, dtz, h, field(a, 2), field(b, 0),   \
