@@ -11,7 +11,8 @@
 // Acoustic, order 8, nbc 50, us per step, cell-per-thread / this: 700x600 16.8 / 12.9, 1000x800
 // 22.7 / 14.2, 1400x1000 31.5 / 17.8, 2000x1600 68.2 / 37.3 (4.6 TB/s of the 48 B that the two half
 // steps move per cell; the working set of 130 MB is just over L2), 8 shots of 600x500
-// 63.9 / 42.0.
+// 63.9 / 42.0.  Elastic: 700x600 24.5 / 18.2, 1000x800 34.9 / 22.0, 1400x1000 65.8 / 31.3,
+// 2000x1600 157 / 67.5.  Scalar: 1000x800 10.9 / 6.8, 2000x1600 25.9 / 17.6.
 #pragma once
 #include "resident2d.cuh"
 
@@ -374,6 +375,366 @@ __global__ void __launch_bounds__(kThreads)
       if (tg.w >= 0) u[3] = tagged(tg.w, e + 3, u[3]);
     }
     stg4(p1 + so + e, u);
+  }
+}
+
+// Pre-correction velocities / stresses of an edge quad (el_vel_at, el_str_at).
+template <int N>
+__device__ __forceinline__ void el_vel_quad(const Geo2& g, const Coef& c, float dtx, float dtz,
+                                            const ElFields& a, const ElMat& m, int x, int z,
+                                            float (&u)[2][4]) {
+  const long long p = (long long)z * g.ld + x;
+  float zx[4], zz[4];
+  {
+    res::Vec<4> w[2 * N];
+    edge_rows<N>(g, a.txz, x, z, N, w);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) zx[j] = __fmul_rn(dtz, res::zdm<N, 4>(w, N, j, c));
+    edge_rows<N>(g, a.tzz, x, z, N - 1, w);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) zz[j] = __fmul_rn(dtz, res::zdp<N, 4>(w, N - 1, j, c));
+  }
+  GWin<N> xw;
+  edge_window<N>(g, a.txx, x, z, xw);
+  const res::Vec<4> ox = ldg4(a.vx + p), oz = ldg4(a.vz + p), bx = ldg4(m.bx + p),
+                    bz = ldg4(m.bz + p);
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const float v = __fmaf_rn(bx[j], __fmaf_rn(dtx, xw.dm(j, c), zx[j]), ox[j]);
+    u[0][j] = interior2(g, x + j, z) ? v : ox[j];
+  }
+  edge_window<N>(g, a.txz, x, z, xw);
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const float v = __fmaf_rn(bz[j], __fmaf_rn(dtx, xw.dp(j, c), zz[j]), oz[j]);
+    u[1][j] = interior2(g, x + j, z) ? v : oz[j];
+  }
+}
+template <int N>
+__device__ __forceinline__ void el_str_quad(const Geo2& g, const Coef& c, float dtx, float dtz,
+                                            const float* __restrict__ vx,
+                                            const float* __restrict__ vz, const ElFields& a,
+                                            const ElMat& m, int x, int z, float (&u)[3][4]) {
+  const long long p = (long long)z * g.ld + x;
+  float ez[4], sh[4];
+  {
+    res::Vec<4> w[2 * N];
+    edge_rows<N>(g, vz, x, z, N, w);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) ez[j] = __fmul_rn(res::zdm<N, 4>(w, N, j, c), dtz);
+    edge_rows<N>(g, vx, x, z, N - 1, w);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) sh[j] = res::zdp<N, 4>(w, N - 1, j, c);
+  }
+  GWin<N> xw;
+  edge_window<N>(g, vx, x, z, xw);
+  const res::Vec<4> oxx = ldg4(a.txx + p), ozz = ldg4(a.tzz + p), oxz = ldg4(a.txz + p);
+  const res::Vec<4> la = ldg4(m.lam + p), l2 = ldg4(m.l2m + p), mu = ldg4(m.mut + p);
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const float ex = __fmul_rn(xw.dp(j, c), dtx);
+    const bool in = interior2(g, x + j, z);
+    u[0][j] = in ? __fadd_rn(oxx[j], __fmaf_rn(l2[j], ex, __fmul_rn(la[j], ez[j]))) : oxx[j];
+    u[1][j] = in ? __fadd_rn(ozz[j], __fmaf_rn(la[j], ex, __fmul_rn(l2[j], ez[j]))) : ozz[j];
+  }
+  edge_window<N>(g, vz, x, z, xw);
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const float v = __fmaf_rn(mu[j], __fmaf_rn(sh[j], dtz, __fmul_rn(xw.dm(j, c), dtx)), oxz[j]);
+    u[2][j] = interior2(g, x + j, z) ? v : oxz[j];
+  }
+}
+
+template <int N, int R, bool SP>
+__global__ void __launch_bounds__(kThreads)
+    k_el_vel_bulk(Geo2 g, Split s, Coef c, float dtx, float dtz, HabcDev h, ElFields a, ElMat m,
+                  float* __restrict__ vx1, float* __restrict__ vz1) {
+  const long long so = (long long)blockIdx.z * g.plane;
+  a.vx += so; a.vz += so; a.txx += so; a.tzz += so; a.txz += so;
+  int x, z;
+  if ((int)blockIdx.x < s.edge) {
+    const int i = blockIdx.x * kThreads + threadIdx.x;
+    if (i >= s.quads) return;
+    edge_quad(s, i, x, z);
+    float u[2][4];
+    el_vel_quad<N>(g, c, dtx, dtz, a, m, x, z, u);
+    int sz, ex;
+    if constexpr (SP) {
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        u[0][j] = x + j < g.nx ? sponge_damp(g, h, x + j, z, u[0][j]) : 0.0f;
+        u[1][j] = x + j < g.nx ? sponge_damp(g, h, x + j, z, u[1][j]) : 0.0f;
+      }
+    } else if (edge_sides(g, x, z, sz, ex)) {
+      float v[2][4] = {}, e[2] = {};
+      if (sz) el_vel_quad<N>(g, c, dtx, dtz, a, m, x, z + sz, v);
+      if (ex >= 0) el_vel_at<N>(g, c, dtx, dtz, a, m, ex, z, e[0], e[1]);
+      edge_blend<2>(g, h, x, z, sz, {0, 1}, u, v, e, {a.vx, a.vz});
+    }
+    const long long p = so + (long long)z * g.ld + x;
+    edge_store(g, vx1 + p, x, u[0]);
+    edge_store(g, vz1 + p, x, u[1]);
+    return;
+  }
+  int rows;
+  if (!inner_cells<R>(s, blockIdx.x - s.edge, x, z, rows)) return;
+  const long long q = (long long)z * g.ld + x;
+  constexpr int NWIN = R + 2 * N - 1;
+  float zx[R][4], zz[R][4];
+  {  // one register window at a time
+    res::Vec<4> w[NWIN];
+#pragma unroll
+    for (int i = 0; i < NWIN; ++i)
+      w[i] = ldg4(a.txz + q + (long long)min(i - N, rows - 1 + N) * g.ld);
+#pragma unroll
+    for (int k = 0; k < R; ++k)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) zx[k][j] = __fmul_rn(dtz, res::zdm<N, 4>(w, N + k, j, c));
+#pragma unroll
+    for (int i = 0; i < NWIN; ++i)
+      w[i] = ldg4(a.tzz + q + (long long)min(i - (N - 1), rows - 1 + N) * g.ld);
+#pragma unroll
+    for (int k = 0; k < R; ++k)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) zz[k][j] = __fmul_rn(dtz, res::zdp<N, 4>(w, N - 1 + k, j, c));
+  }
+#pragma unroll
+  for (int k = 0; k < R; ++k) {
+    if (k >= rows) break;
+    const long long e = q + (long long)k * g.ld;
+    GWin<N> xw;
+    xw.load(a.txx + e);
+    const res::Vec<4> ox = lds4(a.vx + e), oz = lds4(a.vz + e), bx = lds4(m.bx + e),
+                      bz = lds4(m.bz + e);
+    float u[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      u[j] = __fmaf_rn(bx[j], __fmaf_rn(dtx, xw.dm(j, c), zx[k][j]), ox[j]);
+    stg4(vx1 + so + e, u);
+    xw.load(a.txz + e);
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      u[j] = __fmaf_rn(bz[j], __fmaf_rn(dtx, xw.dp(j, c), zz[k][j]), oz[j]);
+    stg4(vz1 + so + e, u);
+  }
+}
+
+// TG: inject into txx, tzz and record vx, vz on tagged cells (step *t.it0 + j0 + 1).
+template <int N, int R, bool SP, bool TG>
+__global__ void __launch_bounds__(kThreads)
+    k_el_str_bulk(Geo2 g, Split s, Coef c, float dtx, float dtz, HabcDev h, ElFields a,
+                  const float* __restrict__ vx1, const float* __restrict__ vz1, ElMat m,
+                  float* __restrict__ txx1, float* __restrict__ tzz1, float* __restrict__ txz1,
+                  CellTags t, int j0) {
+  const long long so = (long long)blockIdx.z * g.plane;
+  a.txx += so; a.tzz += so; a.txz += so;
+  vx1 += so;
+  vz1 += so;
+  auto tagged = [&](int e, long long p, float& sxx, float& szz) {
+    const long long k = (long long)(*t.it0 + j0);
+    const int4 E = t.ent[e];
+    sxx = tag_inject(t, E, k, blockIdx.z, sxx);
+    szz = tag_inject(t, E, k, blockIdx.z, szz);
+    tag_record(t, E, k, blockIdx.z, __ldg(vx1 + p), __ldg(vz1 + p), 0.0f);
+  };
+  int x, z;
+  if ((int)blockIdx.x < s.edge) {
+    const int i = blockIdx.x * kThreads + threadIdx.x;
+    if (i >= s.quads) return;
+    edge_quad(s, i, x, z);
+    float u[3][4];
+    el_str_quad<N>(g, c, dtx, dtz, vx1, vz1, a, m, x, z, u);
+    int sz, ex;
+    if constexpr (SP) {
+#pragma unroll
+      for (int f = 0; f < 3; ++f)
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+          u[f][j] = x + j < g.nx ? sponge_damp(g, h, x + j, z, u[f][j]) : 0.0f;
+    } else if (edge_sides(g, x, z, sz, ex)) {
+      float v[3][4] = {}, e[3] = {};
+      if (sz) el_str_quad<N>(g, c, dtx, dtz, vx1, vz1, a, m, x, z + sz, v);
+      if (ex >= 0) el_str_at<N>(g, c, dtx, dtz, vx1, vz1, a, m, ex, z, e[0], e[1], e[2]);
+      edge_blend<3>(g, h, x, z, sz, {2, 2, 2}, u, v, e, {a.txx, a.tzz, a.txz});
+    }
+    const long long p = (long long)z * g.ld + x;
+    if constexpr (TG) {
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        if (x + j < g.nx) {
+          const int e = __ldg(t.tag + p + j);
+          if (e >= 0) tagged(e, p + j, u[0][j], u[1][j]);
+        }
+    }
+    edge_store(g, txx1 + so + p, x, u[0]);
+    edge_store(g, tzz1 + so + p, x, u[1]);
+    edge_store(g, txz1 + so + p, x, u[2]);
+    return;
+  }
+  int rows;
+  if (!inner_cells<R>(s, blockIdx.x - s.edge, x, z, rows)) return;
+  const long long q = (long long)z * g.ld + x;
+  constexpr int NWIN = R + 2 * N - 1;
+  float ez[R][4], sh[R][4];
+  {
+    res::Vec<4> w[NWIN];
+#pragma unroll
+    for (int i = 0; i < NWIN; ++i)
+      w[i] = ldg4(vz1 + q + (long long)min(i - N, rows - 1 + N) * g.ld);
+#pragma unroll
+    for (int k = 0; k < R; ++k)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) ez[k][j] = __fmul_rn(res::zdm<N, 4>(w, N + k, j, c), dtz);
+#pragma unroll
+    for (int i = 0; i < NWIN; ++i)
+      w[i] = ldg4(vx1 + q + (long long)min(i - (N - 1), rows - 1 + N) * g.ld);
+#pragma unroll
+    for (int k = 0; k < R; ++k)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) sh[k][j] = res::zdp<N, 4>(w, N - 1 + k, j, c);
+  }
+#pragma unroll
+  for (int k = 0; k < R; ++k) {
+    if (k >= rows) break;
+    const long long e = q + (long long)k * g.ld;
+    GWin<N> xw;
+    xw.load(vx1 + e);
+    float sxx[4], szz[4], sxz[4];
+    {
+      const res::Vec<4> oxx = lds4(a.txx + e), ozz = lds4(a.tzz + e), la = lds4(m.lam + e),
+                        l2 = lds4(m.l2m + e);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const float ex = __fmul_rn(xw.dp(j, c), dtx);
+        sxx[j] = __fadd_rn(oxx[j], __fmaf_rn(l2[j], ex, __fmul_rn(la[j], ez[k][j])));
+        szz[j] = __fadd_rn(ozz[j], __fmaf_rn(la[j], ex, __fmul_rn(l2[j], ez[k][j])));
+      }
+    }
+    xw.load(vz1 + e);
+    const res::Vec<4> oxz = lds4(a.txz + e), mu = lds4(m.mut + e);
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      sxz[j] = __fmaf_rn(mu[j], __fmaf_rn(sh[k][j], dtz, __fmul_rn(xw.dm(j, c), dtx)), oxz[j]);
+    if constexpr (TG) {
+      const int4 tg = __ldg(reinterpret_cast<const int4*>(t.tag + e));
+      if (tg.x >= 0) tagged(tg.x, e, sxx[0], szz[0]);
+      if (tg.y >= 0) tagged(tg.y, e + 1, sxx[1], szz[1]);
+      if (tg.z >= 0) tagged(tg.z, e + 2, sxx[2], szz[2]);
+      if (tg.w >= 0) tagged(tg.w, e + 3, sxx[3], szz[3]);
+    }
+    stg4(txx1 + so + e, sxx);
+    stg4(tzz1 + so + e, szz);
+    stg4(txz1 + so + e, sxz);
+  }
+}
+
+// scalar2d leapfrog (sc_at): u2 from u1, u0.
+template <int N>
+__device__ __forceinline__ float sc_cell(const D2Coef& c, float uc, float u0, float c2,
+                                         const float (&nb)[N]) {
+  float lap = __fmul_rn(c.two_c0, uc);
+#pragma unroll
+  for (int l = 0; l < N; ++l) lap = __fmaf_rn(c.d[l], nb[l], lap);
+  return __fmaf_rn(c2, lap, __fsub_rn(__fmul_rn(2.0f, uc), u0));
+}
+template <int N>
+__device__ __forceinline__ void sc_quad(const Geo2& g, const D2Coef& c,
+                                        const float* __restrict__ u1,
+                                        const float* __restrict__ u0,
+                                        const float* __restrict__ c2, int x, int z,
+                                        float (&u)[1][4]) {
+  using B = res::XWin<N, 4>;
+  const long long p = (long long)z * g.ld + x;
+  const res::Vec<4> o = ldg4(u0 + p), m = ldg4(c2 + p);
+  GWin<N> xw;
+  edge_window<N>(g, u1, x, z, xw);
+  res::Vec<4> a[2 * N], b[1];
+  edge_rows<N>(g, u1, x, z, N, a);  // rows z - N .. z + N - 1
+  b[0] = ldg4(u1 + (long long)min(z + N, g.nz - 1) * g.ld + x);
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    float nb[N];
+#pragma unroll
+    for (int l = 1; l <= N; ++l)
+      nb[l - 1] = __fadd_rn(__fadd_rn(__fadd_rn(xw.w[B::L + j + l], xw.w[B::L + j - l]),
+                                      l == N ? b[0][j] : a[l == N ? 0 : N + l][j]),
+                            a[N - l][j]);
+    const float uc = xw.w[B::L + j];
+    const float v = sc_cell<N>(c, uc, o[j], m[j], nb);
+    u[0][j] = interior2(g, x + j, z) ? v : uc;
+  }
+}
+template <int N, int R, bool TG>
+__global__ void __launch_bounds__(kThreads)
+    k_sc_bulk(Geo2 g, Split s, D2Coef c, HabcDev h, const float* __restrict__ u1,
+              const float* __restrict__ u0, const float* __restrict__ c2, float* __restrict__ u2,
+              CellTags t, int j0) {
+  auto tagged = [&](int e, float u) {
+    const long long k = (long long)(*t.it0 + j0);
+    const int4 E = t.ent[e];
+    u = tag_inject(t, E, k, 0, u);
+    tag_record(t, E, k, 0, u, 0.0f, 0.0f);
+    return u;
+  };
+  int x, z;
+  if ((int)blockIdx.x < s.edge) {
+    const int i = blockIdx.x * kThreads + threadIdx.x;
+    if (i >= s.quads) return;
+    edge_quad(s, i, x, z);
+    float u[1][4];
+    sc_quad<N>(g, c, u1, u0, c2, x, z, u);
+    int sz, ex;
+    if (edge_sides(g, x, z, sz, ex)) {
+      float v[1][4] = {}, e[1] = {};
+      if (sz) sc_quad<N>(g, c, u1, u0, c2, x, z + sz, v);
+      if (ex >= 0) e[0] = sc_at<N>(g, c, u1, u0, c2, ex, z);
+      edge_blend<1>(g, h, x, z, sz, {2}, u, v, e, {u1});
+    }
+    const long long p = (long long)z * g.ld + x;
+    if constexpr (TG) {
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        if (x + j < g.nx) {
+          const int e = __ldg(t.tag + p + j);
+          if (e >= 0) u[0][j] = tagged(e, u[0][j]);
+        }
+    }
+    edge_store(g, u2 + p, x, u[0]);
+    return;
+  }
+  int rows;
+  if (!inner_cells<R>(s, blockIdx.x - s.edge, x, z, rows)) return;
+  const long long q = (long long)z * g.ld + x;
+  constexpr int NWIN = R + 2 * N;
+  res::Vec<4> w[NWIN];
+#pragma unroll
+  for (int i = 0; i < NWIN; ++i) w[i] = ldg4(u1 + q + (long long)min(i - N, rows - 1 + N) * g.ld);
+#pragma unroll
+  for (int k = 0; k < R; ++k) {
+    if (k >= rows) break;
+    const long long e = q + (long long)k * g.ld;
+    GWin<N> xw;
+    xw.load(u1 + e);
+    const res::Vec<4> o = lds4(u0 + e), m = lds4(c2 + e);
+    float u[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      float nb[N];
+#pragma unroll
+      for (int l = 1; l <= N; ++l)
+        nb[l - 1] = __fadd_rn(__fadd_rn(__fadd_rn(xw.w[GWin<N>::L + j + l], xw.w[GWin<N>::L + j - l]),
+                                        w[N + k + l][j]),
+                              w[N + k - l][j]);
+      u[j] = sc_cell<N>(c, w[N + k][j], o[j], m[j], nb);
+    }
+    if constexpr (TG) {
+      const int4 tg = __ldg(reinterpret_cast<const int4*>(t.tag + e));
+      if (tg.x >= 0) u[0] = tagged(tg.x, u[0]);
+      if (tg.y >= 0) u[1] = tagged(tg.y, u[1]);
+      if (tg.z >= 0) u[2] = tagged(tg.z, u[2]);
+      if (tg.w >= 0) u[3] = tagged(tg.w, u[3]);
+    }
+    stg4(u2 + e, u);
   }
 }
 
