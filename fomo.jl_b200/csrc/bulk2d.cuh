@@ -21,6 +21,10 @@ namespace bulk {
 
 constexpr int kW = 128;  // columns of an inner tile: a warp of 4-cell threads
 constexpr int kThreads = 256;
+// CTAs per SM that the acoustic kernels' registers are bounded to: without the bound
+// (2 to 3) too few loads are in flight to cover the latency (64 uneven
+// shots 466 us per step, with 4 349, with 5, which spills, 372).
+constexpr int ac_blocks(int N) { return N <= 4 ? 4 : 3; }
 
 // The inner rectangle [x0, x1) x [z0, z1) (x0, x1 multiples of 4), its tiles, and the
 // quads (4 cells of a row) of the edge rectangles: above and below it (full rows), left
@@ -235,20 +239,19 @@ __device__ __forceinline__ bool inner_cells(const Split& s, int b, int& x, int& 
   return x < s.x1 && rows > 0;
 }
 
-#define FOMO_BULK_AC_VEL                                                                    \
-  Geo2 g, Split s, Coef c, float dtx, float dtz, HabcDev h, const float* __restrict__ p0,   \
-      const float* __restrict__ vx0, const float* __restrict__ vz0,                         \
-      const float* __restrict__ bx, const float* __restrict__ bz, float* __restrict__ vx1,  \
-      float* __restrict__ vz1
+// Block `blk` of the acoustic velocity half step of one shot.
 template <int N, int R, bool SP>
-__global__ void __launch_bounds__(kThreads) k_ac_vel_bulk(FOMO_BULK_AC_VEL) {
-  const long long so = (long long)blockIdx.z * g.plane;
-  p0 += so;
-  vx0 += so;
-  vz0 += so;
+__device__ __forceinline__ void ac_vel_block(int blk, const Geo2& g, const Split& s, const Coef& c,
+                                             float dtx, float dtz, const HabcDev& h,
+                                             const float* __restrict__ p0,
+                                             const float* __restrict__ vx0,
+                                             const float* __restrict__ vz0,
+                                             const float* __restrict__ bx,
+                                             const float* __restrict__ bz,
+                                             float* __restrict__ vx1, float* __restrict__ vz1) {
   int x, z;
-  if ((int)blockIdx.x < s.edge) {
-    const int i = blockIdx.x * kThreads + threadIdx.x;
+  if (blk < s.edge) {
+    const int i = blk * kThreads + threadIdx.x;
     if (i >= s.quads) return;
     edge_quad(s, i, x, z);
     float u[2][4];
@@ -266,13 +269,13 @@ __global__ void __launch_bounds__(kThreads) k_ac_vel_bulk(FOMO_BULK_AC_VEL) {
       if (ex >= 0) ac_vel_at<N>(g, c, dtx, dtz, p0, vx0, vz0, bx, bz, ex, z, e[0], e[1]);
       edge_blend<2>(g, h, x, z, sz, {0, 1}, u, v, e, {vx0, vz0});
     }
-    const long long p = so + (long long)z * g.ld + x;
+    const long long p = (long long)z * g.ld + x;
     edge_store(g, vx1 + p, x, u[0]);
     edge_store(g, vz1 + p, x, u[1]);
     return;
   }
   int rows;
-  if (!inner_cells<R>(s, blockIdx.x - s.edge, x, z, rows)) return;
+  if (!inner_cells<R>(s, blk - s.edge, x, z, rows)) return;
   const long long q = (long long)z * g.ld + x;
   constexpr int NWIN = R + 2 * N - 1;
   res::Vec<4> w[NWIN];  // p rows z - (N - 1) .. (rows past the rectangle are still in the grid)
@@ -292,33 +295,42 @@ __global__ void __launch_bounds__(kThreads) k_ac_vel_bulk(FOMO_BULK_AC_VEL) {
       ux[j] = __fmaf_rn(__fmul_rn(mx[j], dtx), xw.dm(j, c), ox[j]);
       uz[j] = __fmaf_rn(__fmul_rn(mz[j], dtz), res::zdp<N, 4>(w, N - 1 + k, j, c), oz[j]);
     }
-    stg4(vx1 + so + e, ux);
-    stg4(vz1 + so + e, uz);
+    stg4(vx1 + e, ux);
+    stg4(vz1 + e, uz);
   }
 }
-#undef FOMO_BULK_AC_VEL
-
-// TG: inject into p and record p, vx, vz on tagged cells (step *t.it0 + j0 + 1).
-template <int N, int R, bool SP, bool TG>
-__global__ void __launch_bounds__(kThreads)
-    k_ac_prs_bulk(Geo2 g, Split s, Coef c, float dtx, float dtz, HabcDev h,
-                  const float* __restrict__ p0, const float* __restrict__ vx1,
-                  const float* __restrict__ vz1, const float* __restrict__ kappa,
-                  float* __restrict__ p1, CellTags t, int j0) {
+template <int N, int R, bool SP>
+__global__ void __launch_bounds__(kThreads, ac_blocks(N))
+    k_ac_vel_bulk(Geo2 g, Split s, Coef c, float dtx, float dtz, HabcDev h,
+                  const float* __restrict__ p0, const float* __restrict__ vx0,
+                  const float* __restrict__ vz0, const float* __restrict__ bx,
+                  const float* __restrict__ bz, float* __restrict__ vx1,
+                  float* __restrict__ vz1) {
   const long long so = (long long)blockIdx.z * g.plane;
-  p0 += so;
-  vx1 += so;
-  vz1 += so;
+  ac_vel_block<N, R, SP>(blockIdx.x, g, s, c, dtx, dtz, h, p0 + so, vx0 + so, vz0 + so, bx, bz,
+                         vx1 + so, vz1 + so);
+}
+
+// Block `blk` of the pressure half step.  TG: inject into p and record p, vx, vz on tagged
+// cells (step *t.it0 + j0 + 1).
+template <int N, int R, bool SP, bool TG>
+__device__ __forceinline__ void ac_prs_block(int blk, int shot, const Geo2& g, const Split& s,
+                                             const Coef& c, float dtx, float dtz, const HabcDev& h,
+                                             const float* __restrict__ p0,
+                                             const float* __restrict__ vx1,
+                                             const float* __restrict__ vz1,
+                                             const float* __restrict__ kappa,
+                                             float* __restrict__ p1, const CellTags& t, int j0) {
   auto tagged = [&](int e, long long p, float u) {
     const long long k = (long long)(*t.it0 + j0);
     const int4 E = t.ent[e];
-    u = tag_inject(t, E, k, blockIdx.z, u);
-    tag_record(t, E, k, blockIdx.z, u, __ldg(vx1 + p), __ldg(vz1 + p));
+    u = tag_inject(t, E, k, shot, u);
+    tag_record(t, E, k, shot, u, __ldg(vx1 + p), __ldg(vz1 + p));
     return u;
   };
   int x, z;
-  if ((int)blockIdx.x < s.edge) {
-    const int i = blockIdx.x * kThreads + threadIdx.x;
+  if (blk < s.edge) {
+    const int i = blk * kThreads + threadIdx.x;
     if (i >= s.quads) return;
     edge_quad(s, i, x, z);
     float u[1][4];
@@ -343,11 +355,11 @@ __global__ void __launch_bounds__(kThreads)
           if (e >= 0) u[0][j] = tagged(e, p + j, u[0][j]);
         }
     }
-    edge_store(g, p1 + so + p, x, u[0]);
+    edge_store(g, p1 + p, x, u[0]);
     return;
   }
   int rows;
-  if (!inner_cells<R>(s, blockIdx.x - s.edge, x, z, rows)) return;
+  if (!inner_cells<R>(s, blk - s.edge, x, z, rows)) return;
   const long long q = (long long)z * g.ld + x;
   constexpr int NWIN = R + 2 * N - 1;
   res::Vec<4> w[NWIN];  // vz rows z - N ..
@@ -374,8 +386,18 @@ __global__ void __launch_bounds__(kThreads)
       if (tg.z >= 0) u[2] = tagged(tg.z, e + 2, u[2]);
       if (tg.w >= 0) u[3] = tagged(tg.w, e + 3, u[3]);
     }
-    stg4(p1 + so + e, u);
+    stg4(p1 + e, u);
   }
+}
+template <int N, int R, bool SP, bool TG>
+__global__ void __launch_bounds__(kThreads, ac_blocks(N))
+    k_ac_prs_bulk(Geo2 g, Split s, Coef c, float dtx, float dtz, HabcDev h,
+                  const float* __restrict__ p0, const float* __restrict__ vx1,
+                  const float* __restrict__ vz1, const float* __restrict__ kappa,
+                  float* __restrict__ p1, CellTags t, int j0) {
+  const long long so = (long long)blockIdx.z * g.plane;
+  ac_prs_block<N, R, SP, TG>(blockIdx.x, blockIdx.z, g, s, c, dtx, dtz, h, p0 + so, vx1 + so,
+                             vz1 + so, kappa, p1 + so, t, j0);
 }
 
 // Pre-correction velocities / stresses of an edge quad (el_vel_at, el_str_at).

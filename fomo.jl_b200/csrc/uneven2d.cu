@@ -8,9 +8,10 @@
 //   velocity update + fused HABC   (acoustic2d/fused_kernels.jl:27-63, kernels_det.jl)
 //   pressure update + fused HABC   (fused_kernels.jl:86-114)
 //   inject into p, record p/vx/vz  (inject_source.jl:4-24, fused_kernels.jl:137-149)
-// The whole nt-step run is captured once into a CUDA graph and replayed with a
-// single launch.  The tile shape is chosen by timing candidates on the problem
-// itself (cached per problem shape).  Each shot equals a single acoustic2d
+// AUTO runs the half steps in blocks per thread (bulk2d.cuh) in replayed chunks of
+// steps; kernel 2 the fused single sweep; kernel 1 cell-per-thread tiles, the run
+// captured once into a CUDA graph, the tile shape chosen by timing candidates on the
+// problem itself (cached per problem shape).  Each shot equals a single acoustic2d
 // run bit for bit (same per-cell arithmetic as the two-phase kernels).
 #include <algorithm>
 #include <cmath>
@@ -28,6 +29,7 @@
 #include <cuda.h>
 #include <cudaTypedefs.h>
 
+#include "bulk2d.cuh"
 #include "solver2d_kernels.cuh"
 #include "tma.cuh"
 
@@ -94,11 +96,57 @@ __global__ void __launch_bounds__(256) k_uac_prs(const UShot* __restrict__ shots
   B[2 * sh.plane + (long long)z * sh.ld + x] = u;
 }
 
+// The half steps in blocks per thread (bulk2d.cuh) over a flat list of the shots'
+// blocks: the default, see run_uneven.
+constexpr int kUR = 2;  // rows per thread
+struct BShot {
+  bulk::Split split;
+  int block0;  // the shot's first block
+};
+template <int N>
+__global__ void __launch_bounds__(bulk::kThreads, bulk::ac_blocks(N))
+    k_uac_vel_bulk(const UShot* __restrict__ shots, const BShot* __restrict__ bs,
+                   const int* __restrict__ block_shot, float* __restrict__ state,
+                   const float* __restrict__ mat, Coef c, float dtx, float dtz,
+                   const float* __restrict__ wtab, int nbc, int wstride, int set) {
+  const int k = block_shot[blockIdx.x];
+  const UShot& sh = shots[k];
+  const bulk::Split s = bs[k].split;
+  const Geo2 g{sh.nx, sh.nz, sh.ld, N, nbc, sh.plane};
+  const HabcDev h{sh.q, sh.qt, sh.qxt, nbc, wstride, wtab};
+  const float* A = state + sh.st + (long long)set * 3 * g.plane;
+  float* B = state + sh.st + (long long)(1 - set) * 3 * g.plane;
+  const float* m = mat + sh.mat;
+  bulk::ac_vel_block<N, kUR, false>(blockIdx.x - bs[k].block0, g, s, c, dtx, dtz, h,
+                                    A + 2 * g.plane, A, A + g.plane, m, m + g.plane, B,
+                                    B + g.plane);
+}
+template <int N>
+__global__ void __launch_bounds__(bulk::kThreads, bulk::ac_blocks(N))
+    k_uac_prs_bulk(const UShot* __restrict__ shots, const BShot* __restrict__ bs,
+                   const int* __restrict__ block_shot, float* __restrict__ state,
+                   const float* __restrict__ mat, Coef c, float dtx, float dtz,
+                   const float* __restrict__ wtab, int nbc, int wstride, int set) {
+  const int k = block_shot[blockIdx.x];
+  const UShot& sh = shots[k];
+  const bulk::Split s = bs[k].split;
+  const Geo2 g{sh.nx, sh.nz, sh.ld, N, nbc, sh.plane};
+  const HabcDev h{sh.q, sh.qt, sh.qxt, nbc, wstride, wtab};
+  const float* A = state + sh.st + (long long)set * 3 * g.plane;
+  float* B = state + sh.st + (long long)(1 - set) * 3 * g.plane;
+  bulk::ac_prs_block<N, kUR, false, false>(blockIdx.x - bs[k].block0, k, g, s, c, dtx, dtz, h,
+                                           A + 2 * g.plane, B, B + g.plane,
+                                           mat + sh.mat + 2 * g.plane, B + 2 * g.plane, CellTags{},
+                                           0);
+}
+
 // One block per shot: sources in order into p, then p/vx/vz at the receivers.
+// Step it, or *it0 + it inside a replayed chunk (it0 = steps before the chunk).
 __global__ void k_uinject_record(const UShot* __restrict__ shots, float* __restrict__ state,
                                  const int* __restrict__ src_lin, const float* __restrict__ wav,
                                  const int* __restrict__ rec_lin, float* __restrict__ seis, int it,
-                                 int nt, int set_out) {
+                                 int nt, int set_out, const int* __restrict__ it0) {
+  if (it0) it += *it0;
   const UShot& sh = shots[blockIdx.x];
   float* B = state + sh.st + (long long)set_out * 3 * sh.plane;
   float* p = B + 2 * sh.plane;
@@ -695,6 +743,16 @@ void launch_step_n(int N, cudaStream_t st, int nblk, Tile t, const UShot* shots,
   }
 }
 
+template <int N>
+void launch_bulk(cudaStream_t st, int nblk, const UShot* shots, const BShot* bs,
+                 const int* block_shot, float* state, const float* mat, const Coef& c, float dtdh,
+                 const float* wtab, int nbc, int wstride, int set) {
+  k_uac_vel_bulk<N><<<nblk, bulk::kThreads, 0, st>>>(shots, bs, block_shot, state, mat, c, dtdh,
+                                                     dtdh, wtab, nbc, wstride, set);
+  k_uac_prs_bulk<N><<<nblk, bulk::kThreads, 0, st>>>(shots, bs, block_shot, state, mat, c, dtdh,
+                                                     dtdh, wtab, nbc, wstride, set);
+}
+
 int run_uneven(fomo_ctx* ctx, float dh, float dt, int nt, int nbc, int fd_order, int ns,
                const fomo_shot2d* shots, const fomo_opts* opts, fomo_stats* stats) {
   if (!ctx) return FOMO_EARG;
@@ -776,6 +834,21 @@ int run_uneven(fomo_ctx* ctx, float dh, float dt, int nt, int nbc, int fd_order,
     cells += (long long)u.nx * u.nz;
   }
 
+  // ---- AUTO: the half steps in blocks per thread.  Two launches and an inject/record
+  // launch per step, in replayed chunks, against the persistent sweep (kernel = 2 still selects
+  // it): 64 shots of 200..2000 x 200..800 349 / 451 us per step, 16 shots 86 / 138, 2 shots
+  // 14 / 42; the sweep moves 36 instead of 48 bytes per cell but is a serial march per strip.
+  const bool use_bulk = !(opts && opts->kernel != FOMO_KERNEL_AUTO) &&
+                        !std::getenv("FOMO_UNEVEN_TILE") && !std::getenv("FOMO_UNEVEN_SWEEP");
+  std::vector<BShot> bshot(use_bulk ? ns : 0);
+  std::vector<int> block_shot;
+  for (int s = 0; use_bulk && s < ns; ++s) {
+    const Geo2 g{tab[s].nx, tab[s].nz, tab[s].ld, N, zone, tab[s].plane};
+    bshot[s].split = bulk::make_split(g, zone + 1, bulk::kThreads / 32 * kUR);
+    bshot[s].block0 = (int)block_shot.size();
+    block_shot.insert(block_shot.end(), (size_t)bshot[s].split.edge + bshot[s].split.tiles, s);
+  }
+
   // ---- tile shape: FOMO_UNEVEN_TILE="bx,by" pins it, else timed once per shape ----
   int tsel = -1;
   if (const char* env = std::getenv("FOMO_UNEVEN_TILE")) {
@@ -827,6 +900,9 @@ int run_uneven(fomo_ctx* ctx, float dh, float dt, int nt, int nbc, int fd_order,
   const size_t o_maps = ar.take<CUtensorMap>((size_t)kAcMaps * ns);
   const size_t o_segs = ar.take<int4>(max_seg);
   const size_t o_sched = ar.take<int>(4);
+  const size_t o_bshot = ar.take<BShot>(ns);
+  const size_t o_bblk = ar.take<int>(std::max<size_t>(block_shot.size(), 1));
+  const size_t o_it = ar.take<int>(1);
   int rc;
   if ((rc = ensure_workspace(ctx, ar.off))) return rc;
   float* d_state = ws_ptr<float>(ctx, o_state);
@@ -870,7 +946,7 @@ int run_uneven(fomo_ctx* ctx, float dh, float dt, int nt, int nbc, int fd_order,
 
   // ---- fused single sweep (the default from order 4): strip width autotuned ----
   const char* env_sweep = std::getenv("FOMO_UNEVEN_SWEEP");
-  const bool fused = N >= 2 && ac_encoder() && !std::getenv("FOMO_UNEVEN_TILE") &&
+  const bool fused = !use_bulk && N >= 2 && ac_encoder() && !std::getenv("FOMO_UNEVEN_TILE") &&
                      !(opts && opts->kernel == FOMO_KERNEL_TWO_PHASE);
   AcShot* d_ashot = ws_ptr<AcShot>(ctx, o_ashot);
   CUtensorMap* d_maps = ws_ptr<CUtensorMap>(ctx, o_maps);
@@ -1021,7 +1097,7 @@ int run_uneven(fomo_ctx* ctx, float dh, float dt, int nt, int nbc, int fd_order,
     return FOMO_OK;
   };
 
-  if (!fused && tsel < 0) {  // time each tile shape on three steps of the zero state
+  if (!fused && !use_bulk && tsel < 0) {  // time each tile shape on three steps of the zero state
     FOMO_CU(ctx, cudaMemsetAsync(d_state, 0, 4 * off_state, st));
     float best = 1e30f;
     for (int k = 0; k < kNumTiles; ++k) {
@@ -1045,9 +1121,10 @@ int run_uneven(fomo_ctx* ctx, float dh, float dt, int nt, int nbc, int fd_order,
     std::lock_guard<std::mutex> lk(g_umu);
     g_utune[key] = tsel;
   }
-  if (!fused && (rc = upload_tiles(tsel))) return rc;
+  if (!fused && !use_bulk && (rc = upload_tiles(tsel))) return rc;
   const int nblk = (int)tile_shot.size();
-  const Tile t = fused ? Tile{0, 0} : kTiles[tsel];
+  const Tile t = fused ? Tile{0, 0}
+                 : use_bulk ? Tile{bulk::kW, bulk::kThreads / 32 * kUR} : kTiles[tsel];
 
   // ---- zero state, capture the whole run, replay it once ----
   FOMO_CU(ctx, cudaMemsetAsync(d_state, 0, 4 * off_state, st));
@@ -1067,16 +1144,61 @@ int run_uneven(fomo_ctx* ctx, float dh, float dt, int nt, int nbc, int fd_order,
   }
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
+  if (use_bulk) {  // chunks of 32 steps captured once and replayed, the rest launched
+    BShot* d_bs = ws_ptr<BShot>(ctx, o_bshot);
+    int* d_bblk = ws_ptr<int>(ctx, o_bblk);
+    int* d_it = ws_ptr<int>(ctx, o_it);
+    FOMO_CU(ctx, cudaMemcpyAsync(d_tab, tab.data(), sizeof(UShot) * ns, cudaMemcpyHostToDevice, st));
+    FOMO_CU(ctx, cudaMemcpyAsync(d_bs, bshot.data(), sizeof(BShot) * ns, cudaMemcpyHostToDevice, st));
+    FOMO_CU(ctx, cudaMemcpyAsync(d_bblk, block_shot.data(), 4 * block_shot.size(),
+                                 cudaMemcpyHostToDevice, st));
+    FOMO_CU(ctx, cudaMemsetAsync(d_it, 0, sizeof(int), st));
+    auto step = [&](cudaStream_t s2, int it, const int* it0) {
+      const int nb = (int)block_shot.size(), A = (it - 1) & 1;
+#define FOMO_UB(NN)                                                                              \
+  case NN: launch_bulk<NN>(s2, nb, d_tab, d_bs, d_bblk, d_state, d_mat, c, dtdh, d_w, zone,     \
+                           wstride, A);                                                         \
+    break;
+      switch (N) { FOMO_UB(1) FOMO_UB(2) FOMO_UB(3) FOMO_UB(4) FOMO_UB(5) }
+#undef FOMO_UB
+      k_uinject_record<<<ns, 256, 0, s2>>>(d_tab, d_state, d_src, d_wav, d_rec, d_seis, it, nt,
+                                           1 - A, it0);
+    };
+    constexpr int K = 32;
+    const int nchunk = nt >= 2 * K ? nt / K : 0;
+    if (nchunk) {
+      cudaStream_t cs2 = ctx->own_stream;  // the caller's stream may be uncapturable
+      FOMO_CU(ctx, cudaStreamBeginCapture(cs2, cudaStreamCaptureModeThreadLocal));
+      for (int j = 1; j <= K; ++j) step(cs2, j, d_it);
+      k_step_add<<<1, 1, 0, cs2>>>(d_it, K);
+      cudaError_t ce = cudaStreamEndCapture(cs2, &graph);
+      if (ce == cudaSuccess) ce = cudaGraphInstantiate(&exec, graph, 0);
+      if (graph) cudaGraphDestroy(graph);
+      if (ce != cudaSuccess) return cuda_fail(ctx, ce, "capture of the uneven-batch chunk");
+    }
+    cudaError_t ce = cudaEventRecord(ctx->ev0, st);
+    for (int k = 0; ce == cudaSuccess && k < nchunk; ++k) ce = cudaGraphLaunch(exec, st);
+    for (int it = nchunk * K + 1; it <= nt; ++it) step(st, it, nullptr);
+    if (ce == cudaSuccess) ce = cudaGetLastError();
+    if (ce == cudaSuccess) ce = cudaEventRecord(ctx->ev1, st);
+    if (ce == cudaSuccess) ce = cudaStreamSynchronize(st);
+    if (exec) {
+      cudaStreamSynchronize(st);
+      cudaGraphExecDestroy(exec);
+    }
+    if (ce != cudaSuccess) return cuda_fail(ctx, ce, "uneven-batch steps");
+    FOMO_CU(ctx, cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1));
+  }
   // Capture on the context's own stream: the caller's stream may be the
   // legacy default stream, which cannot be captured.  Replay on the caller's.
   const cudaStream_t cs = ctx->own_stream;
-  if (!fused) {  // velocity / pressure kernels: the run captured into one graph
+  if (!fused && !use_bulk) {  // velocity / pressure kernels: the run captured into one graph
     FOMO_CU(ctx, cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal));
     for (int it = 1; it <= nt; ++it) {
       const int A = (it - 1) & 1;
       launch_step_n(N, cs, nblk, t, d_tab, d_tiles, d_state, d_mat, c, dtdh, d_w, zone, wstride, A);
       k_uinject_record<<<ns, 256, 0, cs>>>(d_tab, d_state, d_src, d_wav, d_rec, d_seis, it, nt,
-                                           1 - A);
+                                           1 - A, nullptr);
     }
     cudaError_t ce = cudaStreamEndCapture(cs, &graph);
     if (ce != cudaSuccess) return cuda_fail(ctx, ce, "capture of the uneven-batch run");

@@ -496,9 +496,10 @@ def acoustic2d_uneven(vps, rhos, dh, dt, nt, f0, *, sx, sz, rx, rz, nbc: int = 5
     receiver indices; ``v_ref``: None (each shot's min positive vp), a number,
     or one value per shot.  Each shot's seismograms equal ``acoustic2d`` on
     that shot (equations/acoustic2d/acoustic2d.jl:47-192) bit for bit.
-    ``kernel``: 0 = the fused single sweep from order 4 (one launch per step
-    for all shots), 1 = velocity and pressure kernels per step.  ``stats.tile``
-    is (threads per strip, 0) for the sweep, the (x, z) block for two kernels.
+    ``kernel``: 0 = velocity and pressure kernels in blocks per thread, 2 = the
+    fused single sweep (from order 4), 1 = cell-per-thread velocity and pressure
+    kernels.  ``stats.tile`` is (threads per strip, 0) for the sweep, the (x, z)
+    block for two kernels.
     """
     ns = len(vps)
     if ns == 0 or len(rhos) != ns or len(sx) != ns or len(sz) != ns or len(rx) != ns \
