@@ -599,10 +599,17 @@ cudaError_t fused3_make_plan(Fused3Plan& p, const Geo3& g, int N, bool elastic, 
   // Persistent CTAs: one per SM for the elastic phases (a CTA holds an SM's
   // registers and most of its shared memory), two for the acoustic ones where
   // they fit; at least 16 planes of work each.  The segment list
-  // runs through the tiles in order, whole z columns, so the tiles marching
-  // side by side are neighbours and read each other's halo rows from L2; the
-  // last wave of tiles is cut into four z chunks (chunk-major) so that the
-  // CTAs finish together.
+  // runs through the tiles in order, so the tiles marching
+  // side by side are neighbours and read each other's halo rows from L2.
+  // Every tile is cut into ten z chunks (chunk-major), so that few tiles still give
+  // each CTA work and all finish together: acoustic grids while the list fits its table
+  // (526 tiles), elastic ones up to 9/8 tiles per CTA.  Chunks of under five planes cost
+  // their pipeline's fill.  Above that the tiles are whole columns and only the last wave
+  // is cut, in four.  us per step, last wave in four -> all in ten (layers included, order 8):
+  //   acoustic 249x238x209 (153 tiles) 461 -> 404, 128x118x138 157 -> 113,
+  //   328x328x268 (264) 790 -> 743, 388x388x288 (364) 1184 -> 1041;
+  //   elastic 148x148x128 (55 tiles) 253 -> 216, 249x238x209 (153) 828 -> 793, order 10
+  //   310x270x250 (220) 1296 -> 1298, 368x368x268 (351) 1849 -> 1899.
   const int ntiles = p.ntx * p.nty;
   const int zlo = g.zlo, zhi = g.zhi, nzo = zhi - zlo;  // planes updated
   if (zlo < 0 || zhi > g.nz || nzo < 1 || g.gnz < g.nz || g.z0 < 0 || g.z0 + g.nz > g.gnz)
@@ -618,9 +625,12 @@ cudaError_t fused3_make_plan(Fused3Plan& p, const Geo3& g, int N, bool elastic, 
   p.grid_v = grid_of(pv);
   p.grid_s = grid_of(ps);
   const int G = std::max(p.grid_v, p.grid_s);
-  const int L = std::min(ntiles, G), K = nzo >= 64 ? 4 : 1;
-  std::vector<int4> segs;
-  segs.reserve((size_t)ntiles + 3 * (size_t)L);
+  const int nall = std::min(10, nzo / 5);
+  const bool all = nall > 1 && (elastic ? 8LL * ntiles <= 9LL * G
+                                        : (long long)nall * ntiles <= ntiles + 4LL * kMaxGrid3);
+  const int L = all ? ntiles : std::min(ntiles, G), K = all ? nall : nzo >= 64 ? 4 : 1;
+  std::vector<int4> segs;  // at most what fused3_table_bytes holds
+  segs.reserve((size_t)(ntiles - L) + (size_t)K * (size_t)L);
   for (int tile = 0; tile < ntiles - L; ++tile)
     segs.push_back(make_int4(tile % p.ntx, tile / p.ntx, zlo, zhi));
   for (int k = 0; k < K; ++k) {
