@@ -74,7 +74,7 @@ __global__ void k_pack(const float* __restrict__ P, uint32_t* __restrict__ F) {
   const float* W1 = P;
   const float* W2 = P + kNW1;
   const float* W3 = P + kNW1 + kNW2;
-  for (int i = threadIdx.x; i < kNFrag / 2; i += blockDim.x) {
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < kNFrag / 2; i += gridDim.x * blockDim.x) {
     int part, base;
     if (i < kOffF2 / 2) { part = 0; base = kOffF1 / 2; }
     else if (i < kOffF3 / 2) { part = 1; base = kOffF2 / 2; }
@@ -104,65 +104,140 @@ __global__ void k_pack(const float* __restrict__ P, uint32_t* __restrict__ F) {
   }
 }
 
-// 3x3 "same" convolution, zero padding.  A block = 4 warps x 16 pixels of one
-// row.  MODE 0: ReLU -> bf16 (16 ch); 1: linear, channel 0 -> fp32;
+// Tile storage of 32-byte pixels in shared memory: the two 16-byte channel halves of pixel
+// column j change places every four pixels, so the eight rows of an ldmatrix (eight
+// neighbouring pixels) fall into different banks.
+__device__ __forceinline__ int tile_at(int pix, int j, int half) {
+  return pix * 32 + ((half ^ ((j >> 2) & 1)) << 4);
+}
+template <bool TRANS>
+__device__ __forceinline__ void ldsm4(uint32_t (&r)[4], const char* p) {
+  const uint32_t a = (uint32_t)__cvta_generic_to_shared(p);
+  if (TRANS)
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(a) : "memory");
+  else
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(a) : "memory");
+}
+// Eight channels of a pixel.  Features come from the caller and may lie on any 4-byte
+// boundary: vec says that they lie on a 16-byte one.
+__device__ __forceinline__ uint4 ld8(const uint16_t* p, int vec) {
+  if (vec) return __ldg(reinterpret_cast<const uint4*>(p));
+  const uint32_t* q = reinterpret_cast<const uint32_t*>(p);
+  return make_uint4(__ldg(q), __ldg(q + 1), __ldg(q + 2), __ldg(q + 3));
+}
+
+// 3x3 "same" convolution, zero padding.  A block = 4 warps of 16 pixels in R rows; its
+// (R + 2) x 66 input pixels are staged once and an A fragment (16 pixels of an input row,
+// one dx) feeds the output rows above, at and below it, each output's taps still in order
+// 0..8.  The layers are bound by their 32 bytes a pixel through L2 and by latency: with one
+// row a block, fragments were loaded nine times from global memory and the weights staged
+// per 64 pixels (32 windows of 64x64: 10.5 -> 7.8 us a layer, 12.6 -> 9.7 with the mask).
+// XC = 16: x has kC channels; 1: one channel a pixel, the others zero (dY of the last layer).
+// MODE 0: ReLU -> bf16 (16 ch); 1: linear, channel 0 -> fp32;
 // 2: multiply by (act > 0) (ReLU derivative of the layer input) -> bf16.
-template <int NT, int MODE>
-__global__ void __launch_bounds__(128) k_conv(int H, int W, const uint16_t* __restrict__ x,
+template <int NT, int MODE, int XC, int R>
+__global__ void __launch_bounds__(128, 4) k_conv(int H, int W, const uint16_t* __restrict__ x, int vec,
                                               const uint32_t* __restrict__ frag,
                                               const uint16_t* __restrict__ act, void* out) {
-  __shared__ uint32_t sf[9 * NT * 64];
-  for (int i = threadIdx.x; i < 9 * NT * 64; i += 128) sf[i] = frag[i];
-  __syncthreads();
+  constexpr int kPW = 66;
+  __shared__ __align__(16) char tile[XC == 1 ? 16 : (R + 2) * kPW * 32];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-  const int x0 = (blockIdx.x * 4 + warp) * 16;
-  const int y = blockIdx.y;
+  const int xb0 = blockIdx.x * 64, x0 = xb0 + warp * 16;
+  const int y0 = blockIdx.y * R;
   const long long img = (long long)blockIdx.z * H * W;
-  if (x0 >= W) return;
-  float acc[NT][4];
-#pragma unroll
-  for (int nt = 0; nt < NT; ++nt) acc[nt][0] = acc[nt][1] = acc[nt][2] = acc[nt][3] = 0.0f;
-#pragma unroll
-  for (int tap = 0; tap < 9; ++tap) {
-    const int yy = y + tap / 3 - 1, dx = tap % 3 - 1;
-    const bool rok = yy >= 0 && yy < H;
-    const int xa = x0 + g + dx, xb = xa + 8;
-    const uint16_t* row = x + (img + (long long)yy * W) * kC;
-    auto ld = [&](int xx, int ch) -> uint32_t {
-      return (rok && xx >= 0 && xx < W) ? __ldg(reinterpret_cast<const uint32_t*>(row + xx * kC + ch))
-                                        : 0u;
-    };
-    const uint32_t a0 = ld(xa, 2 * t), a1 = ld(xb, 2 * t), a2 = ld(xa, 2 * t + 8),
-                   a3 = ld(xb, 2 * t + 8);
-#pragma unroll
-    for (int nt = 0; nt < NT; ++nt) {
-      const uint32_t* b = sf + ((tap * NT + nt) * 32 + lane) * 2;
-      mma_bf16(acc[nt], a0, a1, a2, a3, b[0], b[1]);
+  if (XC == kC) {
+    for (int i = threadIdx.x; i < (R + 2) * kPW * 2; i += 128) {
+      const int q = i >> 1, half = i & 1, row = q / kPW, j = q - row * kPW;
+      const int yy = y0 + row - 1, xx = xb0 + j - 1;
+      uint4 v = make_uint4(0u, 0u, 0u, 0u);
+      if (yy >= 0 && yy < H && xx >= 0 && xx < W)
+        v = ld8(x + (img + (long long)yy * W + xx) * kC + half * 8, vec);
+      *reinterpret_cast<uint4*>(tile + tile_at(q, j, half)) = v;
     }
   }
-  const int pa = x0 + g, pb = pa + 8;
+  uint2 b[9][NT];
 #pragma unroll
-  for (int half = 0; half < 2; ++half) {
-    const int px = half ? pb : pa;
-    if (px >= W) continue;
-    const long long pix = img + (long long)y * W + px;
-    if (MODE == 1) {
-      if (t == 0) reinterpret_cast<float*>(out)[pix] = acc[0][2 * half];
-      continue;
-    }
+  for (int tap = 0; tap < 9; ++tap)
 #pragma unroll
-    for (int nt = 0; nt < NT; ++nt) {
-      const int co = nt * 8 + 2 * t;
-      float v0 = acc[nt][2 * half], v1 = acc[nt][2 * half + 1];
-      if (MODE == 0) {
-        v0 = fmaxf(v0, 0.0f);
-        v1 = fmaxf(v1, 0.0f);
-      } else {
-        const uint32_t a = *reinterpret_cast<const uint32_t*>(act + pix * kC + co);
-        if (!(bf((uint16_t)(a & 0xffffu)) > 0.0f)) v0 = 0.0f;
-        if (!(bf((uint16_t)(a >> 16)) > 0.0f)) v1 = 0.0f;
+    for (int nt = 0; nt < NT; ++nt)
+      b[tap][nt] = __ldg(reinterpret_cast<const uint2*>(frag) + (tap * NT + nt) * 32 + lane);
+  // the layer input whose sign masks the result, fetched with the tile
+  uint32_t m[R][2][NT];
+  if (MODE == 2) {
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+#pragma unroll
+      for (int half = 0; half < 2; ++half) {
+        const int y = y0 + r, px = x0 + g + 8 * half;
+        const uint32_t* a =
+            reinterpret_cast<const uint32_t*>(act + (img + (long long)y * W + px) * kC) + t;
+#pragma unroll
+        for (int nt = 0; nt < NT; ++nt) m[r][half][nt] = y < H && px < W ? __ldg(a + nt * 4) : 0u;
       }
-      reinterpret_cast<uint32_t*>(out)[(pix * kC + co) / 2] = pack2(v0, v1);
+  }
+  if (XC == kC) __syncthreads();
+  if (x0 >= W) return;
+  float acc[R][NT][4];
+#pragma unroll
+  for (int r = 0; r < R; ++r)
+#pragma unroll
+    for (int nt = 0; nt < NT; ++nt)
+      acc[r][nt][0] = acc[r][nt][1] = acc[r][nt][2] = acc[r][nt][3] = 0.0f;
+#pragma unroll
+  for (int row = 0; row < R + 2; ++row) {
+#pragma unroll
+    for (int dx = 0; dx < 3; ++dx) {
+      uint32_t a[4] = {0u, 0u, 0u, 0u};
+      if (XC == kC) {
+        const int j = warp * 16 + dx + (lane & 15);
+        ldsm4<false>(a, tile + tile_at(row * kPW + j, j, lane >> 4));
+      } else {
+        const int yy = y0 + row - 1, xa = x0 + g + dx - 1, xb = xa + 8;
+        const uint16_t* p = x + img + (long long)yy * W;
+        if (t == 0 && yy >= 0 && yy < H) {
+          if (xa >= 0 && xa < W) a[0] = __ldg(p + xa);
+          if (xb < W) a[1] = __ldg(p + xb);
+        }
+      }
+#pragma unroll
+      for (int dy = 0; dy < 3; ++dy) {
+        const int r = row - dy;
+        if (r < 0 || r >= R) continue;
+#pragma unroll
+        for (int nt = 0; nt < NT; ++nt)
+          mma_bf16(acc[r][nt], a[0], a[1], a[2], a[3], b[dy * 3 + dx][nt].x, b[dy * 3 + dx][nt].y);
+      }
+    }
+  }
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    const int y = y0 + r;
+    if (y >= H) break;
+#pragma unroll
+    for (int half = 0; half < 2; ++half) {
+      const int px = x0 + g + 8 * half;
+      if (px >= W) continue;
+      const long long pix = img + (long long)y * W + px;
+      if (MODE == 1) {
+        if (t == 0) reinterpret_cast<float*>(out)[pix] = acc[r][0][2 * half];
+        continue;
+      }
+#pragma unroll
+      for (int nt = 0; nt < NT; ++nt) {
+        const int co = nt * 8 + 2 * t;
+        float v0 = acc[r][nt][2 * half], v1 = acc[r][nt][2 * half + 1];
+        if (MODE == 0) {
+          v0 = fmaxf(v0, 0.0f);
+          v1 = fmaxf(v1, 0.0f);
+        } else {
+          const uint32_t a = m[r][half][nt];
+          if (!(bf((uint16_t)(a & 0xffffu)) > 0.0f)) v0 = 0.0f;
+          if (!(bf((uint16_t)(a >> 16)) > 0.0f)) v1 = 0.0f;
+        }
+        reinterpret_cast<uint32_t*>(out)[(pix * kC + co) / 2] = pack2(v0, v1);
+      }
     }
   }
 }
@@ -170,84 +245,153 @@ __global__ void __launch_bounds__(128) k_conv(int H, int W, const uint16_t* __re
 // Weight gradient partials: block b sums k-steps [b*ks_per, (b+1)*ks_per) of 16
 // pixels (W % 16 == 0, so a k-step is 16 pixels of one row).
 // D[m = ci][n = co] += A[ci][p] B[p][co],  A[ci][p] = X[p + tap, ci],  B = dY.
+// Twelve warps: four share the k-steps, three the rows of taps.  A warp stages its 18 pixels
+// of X and 16 of dY in 16-byte words, two k-steps ahead in registers, and ldmatrix.trans
+// turns pixels into the K dimension (before: one warp for all nine taps, 72 two-byte loads
+// a lane and k-step; 32 windows of 64x64: 32 -> 13 us a layer).
+// NT = 2: dY has kC channels; 1: one channel a pixel.
 template <int NT>
-__global__ void __launch_bounds__(128) k_wgrad(int H, int W, long long nks, int ks_per,
-                                               const uint16_t* __restrict__ x,
+__global__ void __launch_bounds__(384) k_wgrad(int H, int W, long long nks, int ks_per,
+                                               const uint16_t* __restrict__ x, int vec,
                                                const uint16_t* __restrict__ dy,
                                                float* __restrict__ partial) {
-  constexpr int NO = 8 * NT;
-  __shared__ float red[4][9 * 16 * NO];
+  constexpr int NO = 8 * NT, kStage = (18 + 16) * 32;
+  constexpr int kRed = 4 * 9 * 16 * NO * 4;
+  __shared__ __align__(16) char sm[kRed > 12 * kStage ? kRed : 12 * kStage];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-  float acc[9][NT][4];
+  const int kg = warp / 3, ty = warp % 3;
+  char* sx = sm + warp * kStage;
+  char* sy = sx + 18 * 32;
+  float acc[3][NT][4];
 #pragma unroll
-  for (int k = 0; k < 9; ++k)
+  for (int k = 0; k < 3; ++k)
 #pragma unroll
     for (int nt = 0; nt < NT; ++nt) acc[k][nt][0] = acc[k][nt][1] = acc[k][nt][2] = acc[k][nt][3] = 0.0f;
-  const int wpr = W / 16;  // k-steps per row
-  const long long ks0 = (long long)blockIdx.x * ks_per;
-  const long long ks1 = min(nks, ks0 + ks_per);
-  for (long long ks = ks0 + warp; ks < ks1; ks += 4) {
-    const long long rowid = ks / wpr;  // n*H + y
-    const int x0 = (int)(ks - rowid * wpr) * 16;
-    const int y = (int)(rowid % H);
-    const long long img = (rowid / H) * (long long)H * W;
-    const uint16_t* dyr = dy + (img + (long long)y * W + x0) * kC;
-    uint32_t b[NT][2];
-#pragma unroll
-    for (int nt = 0; nt < NT; ++nt) {
-      const int co = nt * 8 + g;
-      const int k0 = 2 * t;
-      b[nt][0] = (uint32_t)dyr[k0 * kC + co] | ((uint32_t)dyr[(k0 + 1) * kC + co] << 16);
-      b[nt][1] = (uint32_t)dyr[(k0 + 8) * kC + co] | ((uint32_t)dyr[(k0 + 9) * kC + co] << 16);
+  // k-steps fit 32 bits (at most 2^31 pixels a batch); wpr of them a row
+  const unsigned wpr = W / 16, ks0 = blockIdx.x * (unsigned)ks_per;
+  const unsigned ks1 = (unsigned)min(nks, (long long)ks0 + ks_per);
+  struct In {
+    uint4 x0, x1, d;  // halves lane and 32 + lane (lane < 4) of the 36 of X; dY
+  };
+  auto load = [&](unsigned ks, In& in) {
+    in.x0 = in.x1 = in.d = make_uint4(0u, 0u, 0u, 0u);
+    if (ks >= ks1) return;
+    const unsigned row = ks / wpr;  // n*H + y
+    const long long rowid = row;
+    const int x0 = (int)(ks - row * wpr) * 16;
+    const int yy = (int)(row % (unsigned)H) + ty - 1;
+    const uint16_t* xr = x + (rowid + ty - 1) * W * kC;
+    if (yy >= 0 && yy < H) {
+      const int xa = x0 - 1 + (lane >> 1), xb = xa + 16;
+      if (xa >= 0) in.x0 = ld8(xr + (long long)xa * kC + (lane & 1) * 8, vec);
+      if (lane < 4 && xb < W) in.x1 = ld8(xr + (long long)xb * kC + (lane & 1) * 8, vec);
+    }
+    if (NT == 2) {
+      in.d = __ldg(reinterpret_cast<const uint4*>(dy + (rowid * W + x0) * kC) + lane);
+    } else {
+      const uint32_t* q = reinterpret_cast<const uint32_t*>(dy + rowid * W + x0);
+      in.d.x = __ldg(q + t);
+      in.d.y = __ldg(q + t + 4);
+    }
+  };
+  auto step = [&](In& in, unsigned next) {
+    __syncwarp();
+    *reinterpret_cast<uint4*>(sx + tile_at(lane >> 1, lane >> 1, lane & 1)) = in.x0;
+    if (lane < 4)
+      *reinterpret_cast<uint4*>(sx + tile_at(16 + (lane >> 1), 16 + (lane >> 1), lane & 1)) = in.x1;
+    if (NT == 2) *reinterpret_cast<uint4*>(sy + tile_at(lane >> 1, lane >> 1, lane & 1)) = in.d;
+    uint32_t b[4] = {g == 0 ? in.d.x : 0u, g == 0 ? in.d.y : 0u, 0u, 0u};  // (p 0-7, 8-15) of co 0-7, of co 8-15
+    load(next, in);  // into the same registers: a copy would wait for the words here
+    __syncwarp();
+    if (NT == 2) {
+      const int j = lane & 15;
+      ldsm4<true>(b, sy + tile_at(j, j, lane >> 4));
     }
 #pragma unroll
-    for (int tap = 0; tap < 9; ++tap) {
-      const int yy = y + tap / 3 - 1, dx = tap % 3 - 1;
-      const bool rok = yy >= 0 && yy < H;
-      const uint16_t* xr = x + (img + (long long)yy * W) * kC;
-      auto xv = [&](int j, int ci) -> uint32_t {  // X at pixel x0+j shifted by the tap
-        const int xx = x0 + j + dx;
-        return (rok && xx >= 0 && xx < W) ? (uint32_t)xr[xx * kC + ci] : 0u;
-      };
-      const int j0 = 2 * t;
-      const uint32_t a0 = xv(j0, g) | (xv(j0 + 1, g) << 16);
-      const uint32_t a1 = xv(j0, g + 8) | (xv(j0 + 1, g + 8) << 16);
-      const uint32_t a2 = xv(j0 + 8, g) | (xv(j0 + 9, g) << 16);
-      const uint32_t a3 = xv(j0 + 8, g + 8) | (xv(j0 + 9, g + 8) << 16);
+    for (int dx = 0; dx < 3; ++dx) {
+      uint32_t a[4];  // p 0-7 of ci 0-7, 8-15; p 8-15 of ci 0-7, 8-15
+      const int j = dx + (lane >> 4) * 8 + (lane & 7);
+      ldsm4<true>(a, sx + tile_at(j, j, (lane >> 3) & 1));
 #pragma unroll
-      for (int nt = 0; nt < NT; ++nt) mma_bf16(acc[tap][nt], a0, a1, a2, a3, b[nt][0], b[nt][1]);
+      for (int nt = 0; nt < NT; ++nt)
+        mma_bf16(acc[dx][nt], a[0], a[1], a[2], a[3], b[2 * nt], b[2 * nt + 1]);
     }
+  };
+  In in0, in1;
+  load(ks0 + kg, in0);
+  load(ks0 + kg + 4, in1);
+  for (unsigned ks = ks0 + kg; ks < ks1; ks += 8) {
+    step(in0, ks + 8);
+    if (ks + 4 >= ks1) break;
+    step(in1, ks + 12);
   }
   // D fragment: (row g / g+8 = ci, cols 2t, 2t+1 = co within the n-tile)
+  __syncthreads();
+  float* red = reinterpret_cast<float*>(sm);
 #pragma unroll
-  for (int tap = 0; tap < 9; ++tap)
+  for (int dx = 0; dx < 3; ++dx)
 #pragma unroll
     for (int nt = 0; nt < NT; ++nt)
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
-        const int ci = g + (e >> 1) * 8, co = nt * 8 + 2 * t + (e & 1);
-        red[warp][(tap * 16 + ci) * NO + co] = acc[tap][nt][e];
+        const int ci = g + (e >> 1) * 8, co = nt * 8 + 2 * t + (e & 1), tap = ty * 3 + dx;
+        red[((kg * 9 + tap) * 16 + ci) * NO + co] = acc[dx][nt][e];
       }
   __syncthreads();
-  for (int i = threadIdx.x; i < 9 * 16 * NO; i += 128)
-    partial[(long long)blockIdx.x * 9 * 16 * NO + i] =
-        ((red[0][i] + red[1][i]) + red[2][i]) + red[3][i];
+  constexpr int n = 9 * 16 * NO;
+  for (int i = threadIdx.x; i < n; i += 384)
+    partial[(long long)blockIdx.x * n + i] =
+        ((red[i] + red[n + i]) + red[2 * n + i]) + red[3 * n + i];
 }
 
-// Sum the partials in block order into the logical gradient layout.
-__global__ void k_wgrad_reduce(int nblk, int NO, const float* __restrict__ partial, int ci_n,
-                               int co_n, float* __restrict__ grad) {
-  const int n = 9 * ci_n * co_n;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    const int co = i % co_n, ci = (i / co_n) % ci_n, tap = i / (co_n * ci_n);
-    const int j = (tap * 16 + ci) * NO + co;
-    float s = 0.0f;
-    for (int b = 0; b < nblk; ++b) s += partial[(long long)b * 9 * 16 * NO + j];
-    grad[i] = s;
+// Sum the partials in block order into the logical gradient layout, 32 elements a block:
+// 256 threads fetch 128 partials of each at once, one warp adds them in order (a thread's own
+// chain of dependent loads took 16 to 28 us).  The block after the last element's, launched
+// with the loss partials, sums those in order.
+__global__ void __launch_bounds__(256) k_wgrad_reduce(int nblk, int NO,
+                                                      const float* __restrict__ partial, int ci_n,
+                                                      int co_n, float* __restrict__ grad, int nl,
+                                                      const float* __restrict__ lpart, float scale,
+                                                      float* __restrict__ loss) {
+  constexpr int kB = 128;
+  __shared__ float s[kB * 32];
+  const int n = 9 * ci_n * co_n, lane = threadIdx.x & 31, wr = threadIdx.x >> 5;
+  float sum = 0.0f;
+  if ((int)blockIdx.x * 32 >= n) {
+    for (int b0 = 0; b0 < nl; b0 += kB * 32) {
+      const int m = min(kB * 32, nl - b0);
+      __syncthreads();
+      for (int i = threadIdx.x; i < m; i += 256) s[i] = lpart[b0 + i];
+      __syncthreads();
+      if (threadIdx.x == 0) {
+#pragma unroll 16
+        for (int i = 0; i < m; ++i) sum += s[i];
+      }
+    }
+    if (threadIdx.x == 0) *loss = sum * scale;
+    return;
   }
+  const int i = min((int)blockIdx.x * 32 + lane, n - 1);
+  const int co = i % co_n, ci = (i / co_n) % ci_n, tap = i / (co_n * ci_n);
+  const float* p = partial + (tap * 16 + ci) * NO + co;
+  for (int b0 = 0; b0 < nblk; b0 += kB) {
+    const int m = min(kB, nblk - b0);
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < kB / 8; ++k) {
+      const int b = k * 8 + wr;
+      if (b < m) s[b * 32 + lane] = p[(long long)(b0 + b) * 9 * 16 * NO];
+    }
+    __syncthreads();
+    if (wr == 0) {
+#pragma unroll 16
+      for (int b = 0; b < m; ++b) sum += s[b * 32 + lane];
+    }
+  }
+  if (wr == 0 && (int)blockIdx.x * 32 + lane < n) grad[i] = sum;
 }
 
-// Masked mean-square loss: r = m (y - t); dY = 2 r / count (bf16, channel 0);
+// Masked mean-square loss: r = m (y - t); dY = 2 r / count (bf16, one channel);
 // per-block partial sums of r^2 (fixed-order, deterministic).
 __global__ void k_loss(long long npix, const float* __restrict__ y, const float* __restrict__ tgt,
                        const float* __restrict__ mask, float inv_count, uint16_t* __restrict__ dy,
@@ -257,10 +401,7 @@ __global__ void k_loss(long long npix, const float* __restrict__ y, const float*
   for (long long p = blockIdx.x * 256LL + threadIdx.x; p < npix; p += gridDim.x * 256LL) {
     const float r = (mask ? mask[p] : 1.0f) * (y[p] - tgt[p]);
     acc += r * r;
-    uint32_t* d = reinterpret_cast<uint32_t*>(dy + p * kC);
-    d[0] = pack2(2.0f * r * inv_count, 0.0f);
-#pragma unroll
-    for (int k = 1; k < kC / 2; ++k) d[k] = 0u;
+    dy[p] = (uint16_t)pack2(2.0f * r * inv_count, 0.0f);
   }
   s[threadIdx.x] = acc;
   __syncthreads();
@@ -269,14 +410,6 @@ __global__ void k_loss(long long npix, const float* __restrict__ y, const float*
     __syncthreads();
   }
   if (threadIdx.x == 0) part[blockIdx.x] = s[0];
-}
-
-__global__ void k_sum(int n, const float* __restrict__ a, float scale, float* __restrict__ out) {
-  if (threadIdx.x == 0 && blockIdx.x == 0) {
-    float s = 0.0f;
-    for (int i = 0; i < n; ++i) s += a[i];
-    *out = s * scale;
-  }
 }
 
 __global__ void k_adam(int n, float* __restrict__ p, const float* __restrict__ g,
@@ -385,7 +518,7 @@ int plan_bufs(fomo_ctx* ctx, long long npix, int nblk, int nlb, Bufs& b) {
   Arena ar;
   const size_t o_f = ar.take<uint32_t>(kNFrag);
   const size_t o_h1 = ar.take<uint16_t>(npix * kC), o_h2 = ar.take<uint16_t>(npix * kC);
-  const size_t o_d3 = ar.take<uint16_t>(npix * kC), o_dh2 = ar.take<uint16_t>(npix * kC);
+  const size_t o_d3 = ar.take<uint16_t>(npix), o_dh2 = ar.take<uint16_t>(npix * kC);
   const size_t o_dh1 = ar.take<uint16_t>(npix * kC);
   const size_t o_y = ar.take<float>(npix);
   const size_t o_p = ar.take<float>((size_t)std::max(nblk, 1) * 9 * 16 * 16);
@@ -403,13 +536,26 @@ int plan_bufs(fomo_ctx* ctx, long long npix, int nblk, int nlb, Bufs& b) {
   return FOMO_OK;
 }
 
+int aligned16(const void* p) { return reinterpret_cast<uintptr_t>(p) % 16 == 0; }
+
+// Rows per block of a layer: four where that still gives every SM two blocks, else one
+// (a single 120x100 image: 240 blocks of one row, 60 of four).
+template <int NT, int MODE, int XC>
+void conv(cudaStream_t st, int n, int h, int w, const uint16_t* x, const uint32_t* frag,
+          const uint16_t* act, void* out) {
+  const int vec = aligned16(x), wide = (w + 63) / 64, tall = (h + 3) / 4;
+  if ((long long)wide * tall * n >= 296)
+    k_conv<NT, MODE, XC, 4><<<dim3(wide, tall, n), 128, 0, st>>>(h, w, x, vec, frag, act, out);
+  else
+    k_conv<NT, MODE, XC, 1><<<dim3(wide, h, n), 128, 0, st>>>(h, w, x, vec, frag, act, out);
+}
+
 cudaError_t forward(cudaStream_t st, int n, int h, int w, const uint16_t* feat, const float* params,
                     const Bufs& b, float* y, bool pack = true) {
-  if (pack) k_pack<<<1, 256, 0, st>>>(params, b.frag);
-  const dim3 grid((w + 63) / 64, h, n);
-  k_conv<2, 0><<<grid, 128, 0, st>>>(h, w, feat, b.frag + kOffF1, nullptr, b.h1);
-  k_conv<2, 0><<<grid, 128, 0, st>>>(h, w, b.h1, b.frag + kOffF2, nullptr, b.h2);
-  k_conv<1, 1><<<grid, 128, 0, st>>>(h, w, b.h2, b.frag + kOffF3, nullptr, y);
+  if (pack) k_pack<<<(kNFrag / 2 + 255) / 256, 256, 0, st>>>(params, b.frag);
+  conv<2, 0, kC>(st, n, h, w, feat, b.frag + kOffF1, nullptr, b.h1);
+  conv<2, 0, kC>(st, n, h, w, b.h1, b.frag + kOffF2, nullptr, b.h2);
+  conv<1, 1, kC>(st, n, h, w, b.h2, b.frag + kOffF3, nullptr, y);
   return cudaGetLastError();
 }
 
@@ -532,20 +678,21 @@ int fomo_corr_gradients(fomo_ctx* ctx, int32_t n, int32_t h, int32_t w, const ui
   FOMO_CU(ctx, forward(st, n, h, w, feat, params, b, y));
   // loss and dY3
   const float count = (float)npix;  // the loss is a mean over every pixel (mask zeros included)
-  const dim3 grid((w + 63) / 64, h, n);
   k_loss<<<nlb, 256, 0, st>>>(npix, y, target, mask, 1.0f / count, b.d3, b.lpart);
-  k_sum<<<1, 32, 0, st>>>(nlb, b.lpart, 1.0f / count, loss);
   // layer 3: dW3 = sum h2[p+tap] dY3[p];  dH2 = conv_t(dY3, W3) * (h2 > 0)
-  k_wgrad<1><<<nblk, 128, 0, st>>>(h, w, nks, ks_per, b.h2, b.d3, b.part);
-  k_wgrad_reduce<<<2, 128, 0, st>>>(nblk, 8, b.part, 16, 1, grad + kNW1 + kNW2);
-  k_conv<2, 2><<<grid, 128, 0, st>>>(h, w, b.d3, b.frag + kOffT3, b.h2, b.dh2);
+  k_wgrad<1><<<nblk, 384, 0, st>>>(h, w, nks, ks_per, b.h2, 1, b.d3, b.part);
+  k_wgrad_reduce<<<(kNW3 + 31) / 32 + 1, 256, 0, st>>>(nblk, 8, b.part, 16, 1, grad + kNW1 + kNW2,
+                                                       nlb, b.lpart, 1.0f / count, loss);
+  conv<2, 2, 1>(st, n, h, w, b.d3, b.frag + kOffT3, b.h2, b.dh2);
   // layer 2: dW2 = sum h1[p+tap] dPre2[p];  dH1 = conv_t(dPre2, W2) * (h1 > 0)
-  k_wgrad<2><<<nblk, 128, 0, st>>>(h, w, nks, ks_per, b.h1, b.dh2, b.part);
-  k_wgrad_reduce<<<18, 128, 0, st>>>(nblk, 16, b.part, 16, 16, grad + kNW1);
-  k_conv<2, 2><<<grid, 128, 0, st>>>(h, w, b.dh2, b.frag + kOffT2, b.h1, b.dh1);
+  k_wgrad<2><<<nblk, 384, 0, st>>>(h, w, nks, ks_per, b.h1, 1, b.dh2, b.part);
+  k_wgrad_reduce<<<kNW2 / 32, 256, 0, st>>>(nblk, 16, b.part, 16, 16, grad + kNW1, 0, nullptr, 0.0f,
+                                            nullptr);
+  conv<2, 2, kC>(st, n, h, w, b.dh2, b.frag + kOffT2, b.h1, b.dh1);
   // layer 1: dW1 = sum feat[p+tap] dPre1[p]
-  k_wgrad<2><<<nblk, 128, 0, st>>>(h, w, nks, ks_per, feat, b.dh1, b.part);
-  k_wgrad_reduce<<<5, 128, 0, st>>>(nblk, 16, b.part, kCin, 16, grad);
+  k_wgrad<2><<<nblk, 384, 0, st>>>(h, w, nks, ks_per, feat, aligned16(feat), b.dh1, b.part);
+  k_wgrad_reduce<<<kNW1 / 32, 256, 0, st>>>(nblk, 16, b.part, kCin, 16, grad, 0, nullptr, 0.0f,
+                                            nullptr);
   FOMO_CU(ctx, cudaGetLastError());
   return FOMO_OK;
 }
