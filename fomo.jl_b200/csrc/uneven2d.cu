@@ -944,7 +944,7 @@ int run_uneven(fomo_ctx* ctx, float dh, float dt, int nt, int nbc, int fd_order,
   Coef c;
   for (int l = 0; l < 5; ++l) c.a[l] = kFD[N][l];
 
-  // ---- fused single sweep (the default from order 4): strip width autotuned ----
+  // ---- fused single sweep (kernel 2, from order 4): strip width autotuned ----
   const char* env_sweep = std::getenv("FOMO_UNEVEN_SWEEP");
   const bool fused = !use_bulk && N >= 2 && ac_encoder() && !std::getenv("FOMO_UNEVEN_TILE") &&
                      !(opts && opts->kernel == FOMO_KERNEL_TWO_PHASE);

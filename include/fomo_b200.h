@@ -66,7 +66,9 @@ extern "C" {
 
 /* fomo_opts.kernel: time-step kernel family (0 lets the autotuner pick) */
 #define FOMO_KERNEL_AUTO 0
-#define FOMO_KERNEL_TWO_PHASE 1    /* velocity sweep + stress sweep per step      */
+#define FOMO_KERNEL_TWO_PHASE 1    /* velocity sweep + stress sweep per step; runs of */
+                                   /* more than 300 steps on grids that fit on chip   */
+                                   /* are one cooperative launch of the same updates  */
 #define FOMO_KERNEL_SINGLE_SWEEP 2 /* one fused sweep per step (z-marching tiles); */
                                    /* 3D: two TMA-staged half steps per step, each    */
                                    /* with its Higdon boundary fused (AUTO's pick,    */
@@ -185,7 +187,7 @@ FOMO_API int fomo_scalar2d(fomo_ctx* ctx, const fomo_grid2d* g, const float* vp,
  * (equations/acoustic2d/batch.jl:180-261) needs one shared model, so shots on
  * grids of different size are separate acoustic2d calls there.  Here each
  * shot brings its own model and acquisition and all shots step together in
- * one graph-captured run.  Every shot's seismograms equal a single
+ * one run, replayed in chunks of captured steps.  Every shot's seismograms equal a single
  * fomo_acoustic2d run of that shot bit for bit. */
 typedef struct fomo_shot2d {
   int32_t nx, nz;        /* interior grid of this shot                          */
@@ -205,6 +207,8 @@ typedef struct fomo_shot2d {
 } fomo_shot2d;
 
 /* Host arrays only (FOMO_F_DEVICE_PTRS returns FOMO_EUNSUPPORTED); FP32.
+ * opts->kernel: AUTO = half steps in blocks per thread, SINGLE_SWEEP = one persistent
+ * launch of the fused sweep, TWO_PHASE = cell-per-thread tiles; same results.
  * stats->sweep_config = tile width * 1000 + tile height of the chosen tiles. */
 FOMO_API int fomo_acoustic2d_uneven(fomo_ctx* ctx, float dh, float dt, int32_t nt, int32_t nbc,
                                     int32_t fd_order, int32_t n_shots, const fomo_shot2d* shots,

@@ -160,3 +160,26 @@ def test_acoustic2d_batch_on_chip(fomo, both, shots):
     a, b = both(fomo.acoustic2d_batch, vp, rho, 10.0, 1e-3, NT, 15.0, **kw)
     _same(a[0], b[0])
     assert not np.array_equal(a[0].seis_p[..., 0], a[0].seis_p[..., 1])
+
+
+def test_on_the_default_stream(fomo):
+    """A run on chip launched on torch's current (legacy default) stream."""
+    import torch
+
+    from fomo_b200 import _lib as L
+
+    rng = np.random.default_rng(3)
+    vp = rng.uniform(2000, 3500, (90, 60)).astype(np.float32, order="F")
+    rho = rng.uniform(1500, 2500, (90, 60)).astype(np.float32, order="F")
+    kw = dict(sx=[45], sz=[10], rx=np.arange(1, 91, 5), rz=np.full(18, 8), nbc=10, fd_order=8)
+    ctx = L.context(0)
+    ctx.use_torch_stream(torch.cuda.current_stream())
+    try:
+        a = fomo.acoustic2d(vp, rho, 10.0, 1e-3, 400, 15.0, **kw)
+        assert fomo.api.last_stats.gpu_launches < 400
+    finally:
+        ctx.set_stream(None)
+    b = fomo.acoustic2d(vp, rho, 10.0, 1e-3, 400, 15.0, **kw)
+    assert np.array_equal(a.seis_p, b.seis_p)
+    assert np.array_equal(a.seis_vz, b.seis_vz)
+    assert np.abs(a.seis_p).max() > 0
