@@ -601,15 +601,16 @@ cudaError_t fused3_make_plan(Fused3Plan& p, const Geo3& g, int N, bool elastic, 
   // they fit; at least 16 planes of work each.  The segment list
   // runs through the tiles in order, so the tiles marching
   // side by side are neighbours and read each other's halo rows from L2.
-  // Every tile is cut into ten z chunks (chunk-major), so that few tiles still give
-  // each CTA work and all finish together: acoustic grids while the list fits its table
-  // (526 tiles), elastic ones up to 9/8 tiles per CTA.  Chunks of under five planes cost
-  // their pipeline's fill.  Above that the tiles are whole columns and only the last wave
-  // is cut, in four.  us per step, last wave in four -> all in ten (layers included, order 8):
+  // Every tile is cut into ten z chunks (chunk-major) where that gives idle CTAs work or evens
+  // out the last wave: up to 0.7 acoustic or 0.5 elastic tiles per CTA, and if a chunk has 12
+  // planes (its pipeline has to fill) up to 9/8 elastic tiles per CTA and as many acoustic
+  // ones as the list's table holds (526).  Otherwise the tiles are whole columns and only the last wave is cut, in four.
+  // us per step, last wave in four -> all in ten (layers included, order 8):
   //   acoustic 249x238x209 (153 tiles) 461 -> 404, 128x118x138 157 -> 113,
-  //   328x328x268 (264) 790 -> 743, 388x388x288 (364) 1184 -> 1041;
-  //   elastic 148x148x128 (55 tiles) 253 -> 216, 249x238x209 (153) 828 -> 793, order 10
-  //   310x270x250 (220) 1296 -> 1298, 368x368x268 (351) 1849 -> 1899.
+  //   328x328x268 (264) 790 -> 743, 388x388x288 (364) 1184 -> 1041, but in shorter chunks
+  //   548x328x108 (456) 498 -> 528, 428x418x38 (420) 193 -> 213;
+  //   elastic 148x148x128 (55 tiles) 253 -> 216, 249x238x209 (153) 828 -> 793, but 348x168x38
+  //   (144) 151 -> 174, order 10 310x270x250 (220) 1296 -> 1298, 368x368x268 (351) 1849 -> 1899.
   const int ntiles = p.ntx * p.nty;
   const int zlo = g.zlo, zhi = g.zhi, nzo = zhi - zlo;  // planes updated
   if (zlo < 0 || zhi > g.nz || nzo < 1 || g.gnz < g.nz || g.z0 < 0 || g.z0 + g.nz > g.gnz)
@@ -626,8 +627,10 @@ cudaError_t fused3_make_plan(Fused3Plan& p, const Geo3& g, int N, bool elastic, 
   p.grid_s = grid_of(ps);
   const int G = std::max(p.grid_v, p.grid_s);
   const int nall = std::min(10, nzo / 5);
-  const bool all = nall > 1 && (elastic ? 8LL * ntiles <= 9LL * G
-                                        : (long long)nall * ntiles <= ntiles + 4LL * kMaxGrid3);
+  const bool few = elastic ? 2LL * ntiles <= G : 10LL * ntiles <= 7LL * G;
+  const bool tall = nzo >= 120 && (elastic ? 8LL * ntiles <= 9LL * G
+                                           : 10LL * ntiles <= ntiles + 4LL * kMaxGrid3);
+  const bool all = nall > 1 && (few || tall);
   const int L = all ? ntiles : std::min(ntiles, G), K = all ? nall : nzo >= 64 ? 4 : 1;
   std::vector<int4> segs;  // at most what fused3_table_bytes holds
   segs.reserve((size_t)(ntiles - L) + (size_t)K * (size_t)L);

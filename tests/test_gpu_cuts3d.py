@@ -5,11 +5,13 @@ import pytest
 
 pytestmark = pytest.mark.gpu
 
-# one tile in one, two, nine and ten chunks; tiles just below and above the lines of the rule
-SIZES = [("acoustic", 20, 10, 5, 1), ("acoustic", 20, 10, 7, 1), ("acoustic", 25, 9, 41, 1),
-         ("acoustic", 61, 30, 57, 3), ("acoustic", 780, 272, 46, 1), ("acoustic", 780, 290, 46, 1),
-         ("elastic", 20, 10, 5, 1), ("elastic", 20, 10, 7, 1), ("elastic", 61, 30, 57, 3),
-         ("elastic", 350, 170, 22, 2), ("elastic", 380, 170, 22, 2)]
+# few planes, tiles in five to ten chunks, tiles just below and above the lines of the rule
+SIZES = [("acoustic", 20, 10, 5, 1), ("acoustic", 20, 10, 23, 1), ("acoustic", 25, 9, 41, 1),
+         ("acoustic", 61, 30, 57, 3), ("acoustic", 430, 180, 32, 1), ("acoustic", 450, 190, 32, 1),
+         ("acoustic", 780, 270, 122, 1), ("acoustic", 780, 255, 116, 1), ("acoustic", 780, 255, 122, 1),
+         ("elastic", 20, 10, 5, 1), ("elastic", 20, 10, 23, 1), ("elastic", 61, 30, 57, 3),
+         ("elastic", 230, 100, 40, 2), ("elastic", 260, 110, 40, 2), ("elastic", 350, 166, 122, 1),
+         ("elastic", 350, 166, 112, 1), ("elastic", 380, 170, 122, 1)]
 
 
 @pytest.mark.parametrize("order", [2, 8])
