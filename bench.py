@@ -14,7 +14,7 @@ over ranks.
 
 Secondary workloads (one JSON line each, same keys; not the default line):
     --workload elastic-fp16   the same batch with binary16 wavefield storage
-    --workload uneven         64 acoustic shots on grids of uneven size (graph run)
+    --workload uneven         64 acoustic shots on grids of uneven size (replayed chunks)
     --workload elastic3d      elastic3d 400x400x300, nbc 40, order 8 (nt from --nt;
                               --grid3d / --kernel3d: other sizes and kernel forms)
     --workload acoustic3d     acoustic3d on the same model and grid
