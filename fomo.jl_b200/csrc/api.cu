@@ -1,6 +1,5 @@
 // api.cu -- context, errors, workspace and host-side helpers of libfomo_b200.
 #include <algorithm>
-#include <atomic>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
@@ -8,6 +7,7 @@
 #include <vector>
 
 #include "fomo_internal.cuh"
+#include "staging.h"
 
 namespace fomo {
 
@@ -74,7 +74,6 @@ namespace {
 constexpr int kPinSlots = 8;
 constexpr size_t kPinChunk = size_t(4) << 20;
 constexpr int kUploadThreads = 4;
-static_assert(kPinSlots == 2 * kUploadThreads, "each upload thread alternates two slots");
 
 void free_pin(fomo_ctx* ctx) {
   for (auto& e : ctx->pin_ev) {
@@ -119,10 +118,12 @@ void on_threads(int n, F f) {
 
 }  // namespace
 
-// A copy from pageable memory runs through the driver at 11 GB/s; four threads that copy
-// 4 MB chunks into pinned slots keep the bus at its rate (576 MB of 3D models: 52 ms
+// A copy from pageable memory runs through the driver at 11 GB/s; threads that copy 4 MB
+// chunks into pinned slots keep the bus at its rate (576 MB of 3D models: 52 ms
 // direct; elastic3d 400x400x300 spends 113 ms a call on the host before, 27 ms with this and
-// fomo_min_positive).  Pinned sources and small copies go directly.
+// fomo_min_positive).  It pays from where it begins (an acoustic2d call less its loop, two
+// models of 16.0 MB direct 4.6 ms, of 16.8 MB staged 3.6); smaller sizes are not measured.
+// Pinned sources and small copies go directly.
 cudaError_t upload(fomo_ctx* ctx, void* dst, const void* src, size_t bytes, cudaStream_t st) {
   const bool big = bytes >= 4 * kPinChunk;
   cudaPointerAttributes at{};
@@ -132,26 +133,25 @@ cudaError_t upload(fomo_ctx* ctx, void* dst, const void* src, size_t bytes, cuda
   }
   if (!big || at.type != cudaMemoryTypeUnregistered || !ensure_pin(ctx))
     return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, st);
-  const size_t n = (bytes + kPinChunk - 1) / kPinChunk;
-  std::atomic<size_t> next{0};
-  std::atomic<int> err{cudaSuccess};
-  on_threads(kUploadThreads, [&](int w) {
-    cudaError_t e = cudaSetDevice(ctx->device);
-    for (int turn = 0; e == cudaSuccess; ++turn) {
-      const size_t k = next.fetch_add(1);
-      if (k >= n) break;
-      const int slot = 2 * w + (turn & 1);
-      char* p = ctx->pin + slot * kPinChunk;
-      const size_t off = k * kPinChunk, len = std::min(kPinChunk, bytes - off);
-      e = cudaEventSynchronize(ctx->pin_ev[slot]);
-      if (e != cudaSuccess) break;
-      std::memcpy(p, (const char*)src + off, len);
-      e = cudaMemcpyAsync((char*)dst + off, p, len, cudaMemcpyHostToDevice, st);
-      if (e == cudaSuccess) e = cudaEventRecord(ctx->pin_ev[slot], st);
-    }
-    if (e != cudaSuccess) err = e;
-  });
-  return (cudaError_t)err.load();
+  return (cudaError_t)staged_copy(
+      (bytes + kPinChunk - 1) / kPinChunk, kPinSlots, kUploadThreads,
+      [&](size_t slot) -> int {
+        const cudaError_t e = cudaSetDevice(ctx->device);  // a helper's current device is 0
+        return e == cudaSuccess ? cudaEventSynchronize(ctx->pin_ev[slot]) : e;
+      },
+      [&](size_t k, size_t slot) {
+        const size_t off = k * kPinChunk;
+        std::memcpy(ctx->pin + slot * kPinChunk, (const char*)src + off,
+                    std::min(kPinChunk, bytes - off));
+        return 0;
+      },
+      [&](size_t k, size_t slot) -> int {
+        const size_t off = k * kPinChunk;
+        const cudaError_t e =
+            cudaMemcpyAsync((char*)dst + off, ctx->pin + slot * kPinChunk,
+                            std::min(kPinChunk, bytes - off), cudaMemcpyHostToDevice, st);
+        return e == cudaSuccess ? cudaEventRecord(ctx->pin_ev[slot], st) : e;
+      });
 }
 
 // boundary/habc/habc.jl:17-44.  q, qt, qxt in float32 (Float32 arithmetic in
