@@ -383,17 +383,11 @@ int cp_grid(fomo_ctx* ctx, int nx, int nz, int nbc, int fd_order, double sigma, 
   return FOMO_OK;
 }
 
-}  // namespace
-}  // namespace fomo
-
-using namespace fomo;
-
-extern "C" {
-
-int fomo_coupled2d(fomo_ctx* ctx, const fomo_grid2d* gp, const float* vp, const float* vs,
-                   float v_ref_s, double smooth_sigma, const fomo_acq* acq, int32_t snap_interval,
-                   float* seis_P, float* seis_S, float* snaps_P, float* snaps_S,
-                   const fomo_opts* opts, fomo_stats* stats) {
+// on_chip: the run may keep its state on the chip (false: the second try, launched).
+int run_coupled(fomo_ctx* ctx, const fomo_grid2d* gp, const float* vp, const float* vs,
+                float v_ref_s, double smooth_sigma, const fomo_acq* acq, int32_t snap_interval,
+                float* seis_P, float* seis_S, float* snaps_P, float* snaps_S,
+                const fomo_opts* opts, fomo_stats* stats, bool on_chip) {
   if (!ctx) return FOMO_EARG;
   if (!gp || !acq || !vp || !vs)
     return fail(ctx, FOMO_EARG, "grid, acquisition and model arrays are required");
@@ -459,7 +453,7 @@ int fomo_coupled2d(fomo_ctx* ctx, const fomo_grid2d* gp, const float* vp, const 
   // runs that fit keep their state on the chip (resident2d.cuh): 400x300 with nbc 100
   // 15.0 -> 9.7 us per step
   res::Plan rp;
-  if (nt > res::kMinSteps && !(opts && (opts->flags & FOMO_F_STEP_LAUNCH)))
+  if (on_chip && nt > res::kMinSteps && !(opts && (opts->flags & FOMO_F_STEP_LAUNCH)))
     rp = res::make_plan(res::kCoupledNeeds, N, g.nx, g.nz, g.ld, g.nbc, 1,
                         res::sm_count(ctx->device), res::smem_extra(hhp.wstride, 0));
   if (rp.ok) res::plan_entries(rp, 1, tags);
@@ -730,7 +724,10 @@ int fomo_coupled2d(fomo_ctx* ctx, const fomo_grid2d* gp, const float* vp, const 
   if (rp.ok) {
     int hflag = 0;
     FOMO_CU(ctx, cudaMemcpy(&hflag, ctx->d_flag, sizeof(int), cudaMemcpyDeviceToHost));
-    if (hflag) return fail(ctx, FOMO_ECUDA, "on-chip time loop: a bounded halo wait timed out");
+    if (opts && (opts->flags & FOMO_F_ONCHIP_LATE)) hflag = 1;
+    if (hflag)  // a tile gave up on a neighbour's words: launch the steps (run2d does the same)
+      return run_coupled(ctx, gp, vp, vs, v_ref_s, smooth_sigma, acq, snap_interval, seis_P, seis_S,
+                         snaps_P, snaps_S, opts, stats, false);
   }
   float ms = 0.0f;
   FOMO_CU(ctx, cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1));
@@ -748,6 +745,21 @@ int fomo_coupled2d(fomo_ctx* ctx, const fomo_grid2d* gp, const float* vp, const 
     stats->status = FOMO_OK;
   }
   return FOMO_OK;
+}
+
+}  // namespace
+}  // namespace fomo
+
+using namespace fomo;
+
+extern "C" {
+
+int fomo_coupled2d(fomo_ctx* ctx, const fomo_grid2d* gp, const float* vp, const float* vs,
+                   float v_ref_s, double smooth_sigma, const fomo_acq* acq, int32_t snap_interval,
+                   float* seis_P, float* seis_S, float* snaps_P, float* snaps_S,
+                   const fomo_opts* opts, fomo_stats* stats) {
+  return run_coupled(ctx, gp, vp, vs, v_ref_s, smooth_sigma, acq, snap_interval, seis_P, seis_S,
+                     snaps_P, snaps_S, opts, stats, true);
 }
 
 int fomo_debug_coupled_medium(fomo_ctx* ctx, int32_t nx, int32_t nz, int32_t nbc,

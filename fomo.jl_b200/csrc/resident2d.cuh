@@ -16,7 +16,8 @@
 // step k at step k + 2, after it has read its neighbours' words of step k + 1,
 // which they publish only once they have read step k.  Neighbours are mutual:
 // tiles are at least N + 1 cells wide and high.  Every poll is bounded (about a
-// second on the global timer, recorded in *err); after that the tile stops waiting.
+// second on the global timer, recorded in *err); after that the tile stops waiting,
+// and the host runs the steps again as launches, which wait for nobody.
 //
 // What it measured (us per step, order 8, this form / replayed two-phase launches):
 // acoustic 240x200 nbc 50 4.7 / 9.1, 400x300 nbc 100 5.9 / 12.8, 4 shots of 240x200

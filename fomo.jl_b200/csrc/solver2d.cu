@@ -43,6 +43,7 @@ struct Plan2 {
   bool fp16 = false;  // elastic: binary16 wavefield storage (mixed2d.cuh)
   bool sponge = false;  // boundary = :sponge (FOMO_F_SPONGE) instead of HABC
   float sponge_factor = 0.015f;
+  bool on_chip = true;  // may keep its state on the chip (false: the second try, launched)
 };
 
 int check_indices(fomo_ctx* ctx, const char* what, const int32_t* ix, const int32_t* iz,
@@ -391,7 +392,8 @@ int run2d(fomo_ctx* ctx, Plan2& P, const float* vp, const float* vs, const float
   // (resident2d.cuh): AUTO's pick for more than res::kMinSteps steps.
   const bool prof_req = opts && (opts->flags & FOMO_F_PROFILE);
   res::Plan rp;
-  if (P.kernel == FOMO_KERNEL_AUTO && kernel == FOMO_KERNEL_TWO_PHASE && !P.fp16 && !hook && !prof_req && P.nt > res::kMinSteps &&
+  if (P.on_chip && P.kernel == FOMO_KERNEL_AUTO && kernel == FOMO_KERNEL_TWO_PHASE && !P.fp16 &&
+      !hook && !prof_req && P.nt > res::kMinSteps &&
       !(opts && (opts->flags & FOMO_F_STEP_LAUNCH)))
     rp = res::make_plan(P.phys == kAcoustic  ? res::kAcousticNeeds
                         : P.phys == kElastic ? res::kElasticNeeds
@@ -1172,9 +1174,14 @@ int run2d(fomo_ctx* ctx, Plan2& P, const float* vp, const float* vs, const float
   if (kernel == FOMO_KERNEL_SINGLE_SWEEP || rp.ok) {
     int hflag = 0;
     FOMO_CU(ctx, cudaMemcpy(&hflag, ctx->d_flag, sizeof(int), cudaMemcpyDeviceToHost));
-    if (hflag)
-      return fail(ctx, FOMO_ECUDA, rp.ok ? "on-chip time loop: a bounded halo wait timed out"
-                                         : "single-sweep kernel: a bounded TMA wait timed out");
+    if (rp.ok && opts && (opts->flags & FOMO_F_ONCHIP_LATE)) hflag = 1;
+    if (hflag && rp.ok) {
+      // A tile gave up on a neighbour's words: the process was off the GPU for a second
+      // (time slicing, a debugger).  The launched steps wait for nobody: run them instead.
+      P.on_chip = false;
+      return run2d(ctx, P, vp, vs, rho, acq, outs, opts, stats, hook);
+    }
+    if (hflag) return fail(ctx, FOMO_ECUDA, "single-sweep kernel: a bounded TMA wait timed out");
   }
   float ms = 0.0f;
   FOMO_CU(ctx, cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1));

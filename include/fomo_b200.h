@@ -58,6 +58,9 @@ extern "C" {
 #define FOMO_F_SPONGE 8u      /* boundary = :sponge: Cerjan layer of the user's  */
                               /* nbc cells (boundary/sponge.jl) instead of HABC;  */
                               /* acoustic2d and elastic2d (+ batch), FP32 only    */
+/* Failure injection on the host, for tests of the 2D runs that stay on the chip: the run */
+/* is taken to have waited too long for a neighbour tile, and its steps are launched.     */
+#define FOMO_F_ONCHIP_LATE 16u
 
 /* fomo_opts.precision: storage format of wavefields and material arrays */
 #define FOMO_FP32 0
