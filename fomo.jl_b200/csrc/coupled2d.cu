@@ -604,27 +604,25 @@ int run_coupled(fomo_ctx* ctx, const fomo_grid2d* gp, const float* vp, const flo
         f.in[i] = it == 1 ? nullptr : field(A, i);  // the run starts from zero
         f.out[i] = field(B, i);
       }
-      const cudaError_t e = res::launch_coupled(st, N, rp, run, f, cc);
+      const bool refuse = opts && (opts->flags & FOMO_F_ONCHIP_REFUSED);  // injected
+      const cudaError_t e = refuse ? cudaErrorCooperativeLaunchTooLarge
+                                   : res::launch_coupled(st, N, rp, run, f, cc);
       if (it == 1 && e == cudaErrorCooperativeLaunchTooLarge) {
         cudaGetLastError();  // part of the SMs is not ours: launch the steps instead
-        rp.ok = false;
-        chunk_ev.ev.clear();
-        break;
+        return run_coupled(ctx, gp, vp, vs, v_ref_s, smooth_sigma, acq, snap_interval, seis_P,
+                           seis_S, snaps_P, snaps_S, opts, stats, false);
       }
       FOMO_CU(ctx, e);
       launches += 1;
       std::swap(A, B);
       if (stream && run.nsteps == K) FOMO_CU(ctx, cudaEventRecord(chunk_ev.ev[it / K], st));
     }
-    if (rp.ok) {
-      it_first = nt + 1;
-      if (stream) {
-        streamed_chunks = nt / K;
-        frames_per_chunk = K / si;
-      }
+    it_first = nt + 1;
+    if (stream) {
+      streamed_chunks = nt / K;
+      frames_per_chunk = K / si;
     }
-  }
-  if (!rp.ok) {
+  } else {
     const int si = nsnap ? snap_interval : 0;
     int K = 0;
     if (!(opts && (opts->flags & FOMO_F_STEP_LAUNCH))) {

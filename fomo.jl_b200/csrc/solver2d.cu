@@ -761,14 +761,16 @@ int run2d(fomo_ctx* ctx, Plan2& P, const float* vp, const float* vs, const float
       frames_per_chunk = K / si;
     }
     FOMO_CU(ctx, cudaEventRecord(ctx->ev0, st));  // the loop starts after the tables
+    const bool refuse = opts && (opts->flags & FOMO_F_ONCHIP_REFUSED);
     bool first = true;
     for (int it = 1; it <= P.nt; it += run.nsteps) {
       run.it0 = it;
       run.nsteps = std::min(K, P.nt - it + 1);
       res::Fields f{};
       for (int i = 0; i < nmat; ++i) f.mat[i] = d_mat + i * P.plane;
-      cudaError_t e;
-      if (P.phys == kScalar) {  // u^n in set B, u^{n-1} in set A; one launch, from zero
+      cudaError_t e = cudaErrorCooperativeLaunchTooLarge;
+      if (refuse) {  // injected: nothing is launched
+      } else if (P.phys == kScalar) {  // u^n in set B, u^{n-1} in set A; one launch, from zero
         res::Centered cc{};
         cc.c0 = 2.0f * kD2C0[P.N];
         for (int l = 0; l < 5; ++l) cc.d2[l] = kD2[P.N][l];
@@ -785,10 +787,8 @@ int run2d(fomo_ctx* ctx, Plan2& P, const float* vp, const float* vs, const float
       }
       if (first && e == cudaErrorCooperativeLaunchTooLarge) {
         cudaGetLastError();  // part of the SMs is not ours: launch the steps instead
-        rp.ok = false;
-        chunk_ev.ev.clear();
-        frames_per_chunk = 0;
-        break;
+        P.on_chip = false;
+        return run2d(ctx, P, vp, vs, rho, acq, outs, opts, stats, hook);
       }
       FOMO_CU(ctx, e);
       first = false;
@@ -797,13 +797,10 @@ int run2d(fomo_ctx* ctx, Plan2& P, const float* vp, const float* vs, const float
       const int k = it / K;
       if (stream && run.nsteps == K) FOMO_CU(ctx, cudaEventRecord(chunk_ev.ev[k], st));
     }
-    if (rp.ok) {
-      it_first = P.nt + 1;
-      sweeps_per_step = P.phys == kScalar ? 1 : 2;
-      if (stream) streamed_chunks = nchunk;
-    }
-  }
-  if (!rp.ok) {
+    it_first = P.nt + 1;
+    sweeps_per_step = P.phys == kScalar ? 1 : 2;
+    if (stream) streamed_chunks = nchunk;
+  } else {
     const bool scalar = P.phys == kScalar;
     const bool elastic = P.phys == kElastic;
     const bool chunks_ok = (!elastic || kernel == FOMO_KERNEL_TWO_PHASE) && !P.fp16 && !hook &&

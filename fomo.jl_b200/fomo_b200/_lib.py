@@ -25,6 +25,7 @@ FOMO_F_PROFILE = 2
 FOMO_F_STEP_LAUNCH = 4
 FOMO_F_SPONGE = 8
 FOMO_F_ONCHIP_LATE = 16
+FOMO_F_ONCHIP_REFUSED = 32
 FOMO_FP32, FOMO_FP16, FOMO_BF16 = 0, 1, 2
 FOMO_KERNEL_AUTO, FOMO_KERNEL_TWO_PHASE, FOMO_KERNEL_SINGLE_SWEEP = 0, 1, 2
 

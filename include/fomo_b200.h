@@ -59,8 +59,10 @@ extern "C" {
                               /* nbc cells (boundary/sponge.jl) instead of HABC;  */
                               /* acoustic2d and elastic2d (+ batch), FP32 only    */
 /* Failure injection on the host, for tests of the 2D runs that stay on the chip: the run */
-/* is taken to have waited too long for a neighbour tile, and its steps are launched.     */
+/* is taken to have waited too long for a neighbour tile, or its launch to be refused as  */
+/* too large.  The steps are then launched, with the same results.                        */
 #define FOMO_F_ONCHIP_LATE 16u
+#define FOMO_F_ONCHIP_REFUSED 32u
 
 /* fomo_opts.precision: storage format of wavefields and material arrays */
 #define FOMO_FP32 0

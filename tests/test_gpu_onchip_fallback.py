@@ -44,7 +44,7 @@ def _flat(r, fin):
     return out
 
 
-@pytest.mark.parametrize("flag", ["FOMO_F_ONCHIP_LATE"])
+@pytest.mark.parametrize("flag", ["FOMO_F_ONCHIP_LATE", "FOMO_F_ONCHIP_REFUSED"])
 @pytest.mark.parametrize("name", ["acoustic2d", "sponge", "elastic2d", "scalar2d", "coupled2d", "batch"])
 def test_failed_run_on_chip_is_launched(fomo, monkeypatch, name, flag):
     from fomo_b200 import _lib as L
