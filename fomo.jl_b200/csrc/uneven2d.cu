@@ -773,7 +773,7 @@ int run_uneven(fomo_ctx* ctx, float dh, float dt, int nt, int nbc, int fd_order,
   // ---- per-shot validation, geometry and offsets ----
   std::vector<UShot> tab(ns);
   std::vector<int32_t> src_lin, rec_lin;
-  long long off_state = 0, off_mat = 0, off_wav = 0, off_seis = 0, off_model = 0;
+  long long off_state = 0, off_mat = 0, off_wav = 0, off_seis = 0;
   long long cells = 0;
   std::vector<float> wt_ref;
   int wstride = 0, zone = 0;
@@ -830,7 +830,6 @@ int run_uneven(fomo_ctx* ctx, float dh, float dt, int nt, int nbc, int fd_order,
       wstride = hh.wstride;
       zone = hh.nbc;
     }
-    off_model += 2 * nint;
     cells += (long long)u.nx * u.nz;
   }
 
@@ -885,7 +884,6 @@ int run_uneven(fomo_ctx* ctx, float dh, float dt, int nt, int nbc, int fd_order,
   Arena ar;
   const size_t o_state = ar.take<float>(off_state);
   const size_t o_mat = ar.take<float>(off_mat);
-  const size_t o_model = ar.take<float>(off_model);
   const size_t o_wav = ar.take<float>(std::max(off_wav, 1LL));
   const size_t o_seis = ar.take<float>(std::max(off_seis, 1LL));
   const size_t o_src = ar.take<int32_t>(std::max<size_t>(src_lin.size(), 1));
@@ -907,7 +905,6 @@ int run_uneven(fomo_ctx* ctx, float dh, float dt, int nt, int nbc, int fd_order,
   if ((rc = ensure_workspace(ctx, ar.off))) return rc;
   float* d_state = ws_ptr<float>(ctx, o_state);
   float* d_mat = ws_ptr<float>(ctx, o_mat);
-  float* d_model = ws_ptr<float>(ctx, o_model);
   float* d_wav = ws_ptr<float>(ctx, o_wav);
   float* d_seis = ws_ptr<float>(ctx, o_seis);
   int32_t* d_src = ws_ptr<int32_t>(ctx, o_src);
@@ -916,15 +913,15 @@ int run_uneven(fomo_ctx* ctx, float dh, float dt, int nt, int nbc, int fd_order,
   int* d_tiles = ws_ptr<int>(ctx, o_tiles);
   float* d_w = ws_ptr<float>(ctx, o_w);
 
-  // ---- materials per shot (device preparation; every shot has its staging place, so
-  // the shots follow each other without a wait) ----
+  // ---- materials per shot (device preparation).  A shot's raw models are staged in its
+  // own state planes (six padded ones hold two interior ones), which are zeroed before the
+  // first step, so the shots follow each other without a wait and without a buffer of their
+  // own ----
   const float dtdh = dt / dh;
-  long long at_model = 0;
   for (int s = 0; s < ns; ++s) {
     const fomo_shot2d& in = shots[s];
     const long long nint = (long long)in.nx * in.nz;
-    float* raw = d_model + at_model;
-    at_model += 2 * nint;
+    float* raw = d_state + tab[s].st;
     FOMO_CU(ctx, upload(ctx, raw, in.vp, 4 * nint, st));
     FOMO_CU(ctx, upload(ctx, raw + nint, in.rho, 4 * nint, st));
     float* m = d_mat + tab[s].mat;
