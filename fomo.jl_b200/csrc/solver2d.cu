@@ -270,6 +270,22 @@ int tune_sweep(fomo_ctx* ctx, cudaStream_t st, SweepPlan& sp, int N, const Geo2&
 // (10.8 us), at 420 k it falls from 16.8 to 12.9 us.
 constexpr long long kBulkCells = 200000;
 
+// One FP32 elastic shot of a size that AUTO sweeps (pick_kernel_2d): are its two-phase steps
+// in blocks per thread faster?  The one-shot sweep moves fewer bytes but is bound by issue;
+// the blocks' edge quads evaluate two rows, at a cost that grows with the order.  us per step, sweep / blocks, by order, padded cells and the layers'
+// share of them:
+//   order 10:  3.9 M  5 %  100 / 78    5.0 M 10 %  124 / 114   5.9 M  9 %  132 / 132
+//              7.6 M  8 %  159 / 162  12.7 M  6 %  243 / 255  24.9 M  4 %  439 / 461
+//              4.2 M 28 %  111 / 120   6.1 M 16 %  141 / 145  22.9 M 13 %  402 / 472
+//   order 8:   4.0 M 11 %   94 / 78    7.6 M  8 %  145 / 140  20.4 M  2 %  332 / 318
+//              4.1 M 27 %   99 / 102   6.0 M 16 %  120 / 127  22.9 M 13 %  369 / 405
+//   order 4:   4.0 M 10 %   78 / 68    7.6 M  7 %  133 / 124  20.4 M  2 %  307 / 283
+//              4.1 M 27 %   84 / 87    6.0 M 16 %  106 / 110  22.8 M 12 %  341 / 353
+bool blocks_beat_sweep(const Plan2& P) {
+  const double cells = (double)P.nxp * P.nzp, layers = cells - (double)P.nx * P.nz;
+  return layers <= 0.1 * cells && (P.N <= 4 || cells <= 6.0e6);
+}
+
 struct Outs {
   float* seis[3];
   int nseis;
@@ -338,9 +354,8 @@ int run2d(fomo_ctx* ctx, Plan2& P, const float* vp, const float* vs, const float
   if (P.sponge) kernel = FOMO_KERNEL_TWO_PHASE;
   if (kernel == FOMO_KERNEL_AUTO) {
     kernel = pick_kernel_2d((int)P.phys, P.N, P.nxp, P.nzp, P.ns);
-    // one FP32 shot has no pair to sweep, and its two-phase step in blocks per thread is
-    // faster (2000x1600, order 8: 70 us against 87), without the autotuner's first call
-    if (P.ns == 1 && !P.fp16) kernel = FOMO_KERNEL_TWO_PHASE;
+    if (kernel == FOMO_KERNEL_SINGLE_SWEEP && P.ns == 1 && !P.fp16 && blocks_beat_sweep(P))
+      kernel = FOMO_KERNEL_TWO_PHASE;
   }
   if (kernel == FOMO_KERNEL_SINGLE_SWEEP && !sweep2d_supported((int)P.phys, P.N))
     kernel = FOMO_KERNEL_TWO_PHASE;
