@@ -28,6 +28,7 @@
 #include <type_traits>
 #include <vector>
 
+#include "cuts3d.h"
 #include "sweep3d.cuh"
 #include "tma.cuh"
 
@@ -37,7 +38,6 @@ namespace {
 constexpr int kTX = 32, kTY = 16, kNT = kTX * kTY;
 constexpr int kOX = kTX - 2, kOY = kTY - 2;  // output columns / rows of a tile
 constexpr int kCW = 36;                      // centre box width: 32 + up to 3 alignment columns
-constexpr int kMaxGrid3 = 1184;
 
 __host__ __device__ constexpr int al32(int n) { return (n + 31) & ~31; }
 
@@ -579,7 +579,7 @@ bool fused3_supported(int N) { return N >= 1 && N <= 5 && encoder3(); }
 
 size_t fused3_table_bytes(const Geo3& g) {
   const long long ntiles = (long long)((g.nx + kOX - 1) / kOX) * ((g.ny + kOY - 1) / kOY);
-  return (size_t)(ntiles + 4 * kMaxGrid3) * sizeof(int4) + 512;
+  return (size_t)segs3_room(ntiles) * sizeof(int4) + 512;
 }
 
 cudaError_t fused3_make_plan(Fused3Plan& p, const Geo3& g, int N, bool elastic, float* state,
@@ -601,16 +601,7 @@ cudaError_t fused3_make_plan(Fused3Plan& p, const Geo3& g, int N, bool elastic, 
   // they fit; at least 16 planes of work each.  The segment list
   // runs through the tiles in order, so the tiles marching
   // side by side are neighbours and read each other's halo rows from L2.
-  // Every tile is cut into ten z chunks (chunk-major) where that gives idle CTAs work or evens
-  // out the last wave: up to 0.7 acoustic or 0.5 elastic tiles per CTA, and if a chunk has 12
-  // planes (its pipeline has to fill) up to 9/8 elastic tiles per CTA and as many acoustic
-  // ones as the list's table holds (526).  Otherwise the tiles are whole columns and only the last wave is cut, in four.
-  // us per step, last wave in four -> all in ten (layers included, order 8):
-  //   acoustic 249x238x209 (153 tiles) 461 -> 404, 128x118x138 157 -> 113,
-  //   328x328x268 (264) 790 -> 743, 388x388x288 (364) 1184 -> 1041, but in shorter chunks
-  //   548x328x108 (456) 498 -> 528, 428x418x38 (420) 193 -> 213;
-  //   elastic 148x148x128 (55 tiles) 253 -> 216, 249x238x209 (153) 828 -> 793, but 348x168x38
-  //   (144) 151 -> 174, order 10 310x270x250 (220) 1296 -> 1298, 368x368x268 (351) 1849 -> 1899.
+  // How the tiles are cut in z: cuts3d.h.
   const int ntiles = p.ntx * p.nty;
   const int zlo = g.zlo, zhi = g.zhi, nzo = zhi - zlo;  // planes updated
   if (zlo < 0 || zhi > g.nz || nzo < 1 || g.gnz < g.nz || g.z0 < 0 || g.z0 + g.nz > g.gnz)
@@ -626,13 +617,9 @@ cudaError_t fused3_make_plan(Fused3Plan& p, const Geo3& g, int N, bool elastic, 
   p.grid_v = grid_of(pv);
   p.grid_s = grid_of(ps);
   const int G = std::max(p.grid_v, p.grid_s);
-  const int nall = std::min(10, nzo / 5);
-  const bool few = elastic ? 2LL * ntiles <= G : 10LL * ntiles <= 7LL * G;
-  const bool tall = nzo >= 120 && (elastic ? 8LL * ntiles <= 9LL * G
-                                           : 10LL * ntiles <= ntiles + 4LL * kMaxGrid3);
-  const bool all = nall > 1 && (few || tall);
-  const int L = all ? ntiles : std::min(ntiles, G), K = all ? nall : nzo >= 64 ? 4 : 1;
-  std::vector<int4> segs;  // at most what fused3_table_bytes holds
+  const Cuts3 cut = cuts3(elastic, ntiles, nzo, G);
+  const int L = cut.tiles, K = cut.chunks;
+  std::vector<int4> segs;
   segs.reserve((size_t)(ntiles - L) + (size_t)K * (size_t)L);
   for (int tile = 0; tile < ntiles - L; ++tile)
     segs.push_back(make_int4(tile % p.ntx, tile / p.ntx, zlo, zhi));
@@ -642,6 +629,7 @@ cudaError_t fused3_make_plan(Fused3Plan& p, const Geo3& g, int N, bool elastic, 
       segs.push_back(make_int4(tile % p.ntx, tile / p.ntx, z0, z1));
   }
   p.nseg = (int)segs.size();
+  if (p.nseg > segs3_room(ntiles)) return cudaErrorInvalidValue;
   char* tb = static_cast<char*>(d_table);
   p.d_sched = reinterpret_cast<int*>(tb);
   p.d_segs = reinterpret_cast<int4*>(tb + 256);
