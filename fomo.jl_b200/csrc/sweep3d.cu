@@ -617,7 +617,7 @@ cudaError_t fused3_make_plan(Fused3Plan& p, const Geo3& g, int N, bool elastic, 
   p.grid_v = grid_of(pv);
   p.grid_s = grid_of(ps);
   const int G = std::max(p.grid_v, p.grid_s);
-  const Cuts3 cut = cuts3(elastic, ntiles, nzo, G);
+  const Cuts3 cut = cuts3(elastic, ntiles, nzo, G, nsm);
   const int L = cut.tiles, K = cut.chunks;
   std::vector<int4> segs;
   segs.reserve((size_t)(ntiles - L) + (size_t)K * (size_t)L);
