@@ -372,9 +372,11 @@ int run2d(fomo_ctx* ctx, Plan2& P, const float* vp, const float* vs, const float
   // Binary16 batches of two or more shots run the shot-pair sweep's variant of
   // binary16 values in FP32 words (same results, and less memory than a binary16
   // array beside the FP32 band array: 4 bytes per stored value instead of 6);
-  // single shots and a pinned one-shot variant keep binary16 arrays (`half`).
+  // single shots, a pinned one-shot variant and layers too thick for the pair
+  // variant's ramps keep binary16 arrays (`half`).
   const int pinv = pinned_sweep_variant();
-  const bool pair16 = sweep && P.fp16 && P.ns >= 2 && (pinv < 0 || sweep_variant_pair16(pinv));
+  const bool pair16 = sweep && P.fp16 && P.ns >= 2 && pair16_fits(P.N, hh.nbc + 3) &&
+                      (pinv < 0 || sweep_variant_pair16(pinv));
   const bool half = P.fp16 && !pair16;
   const bool pair_ok = sweep && !half && P.phys == kElastic;
   const int nsa = pair_ok ? P.ns + (P.ns & 1) : P.ns;

@@ -103,6 +103,9 @@ struct PairCoef {
 };
 int pair_num_variants();
 bool pair_variant16(int v);  // the variant of binary16 values in FP32 words
+// Whether it fits an SM with ramps of wstride distances (nbc + 3): its four words a distance
+// fill the shared memory at absorbing layers of 2900 to 4000 cells.
+bool pair16_fits(int N, int wstride);
 int pair_threads(int v);
 int pair_txmax(int N, int v);       // widest strip of a variant (even)
 int pair_box_width(int N, int v);   // TMA box width in float2 elements

@@ -681,6 +681,11 @@ int pair_num_variants() { return kNumPair; }
 
 bool pair_variant16(int v) { return v == kPair16; }
 
+bool pair16_fits(int N, int wstride) {
+  const size_t smem = pair_smem(N, kPair16, wstride);
+  return smem <= (size_t)kMaxDynSmemPair && pair_blocks_per_sm(N, kPair16, smem) >= 1;
+}
+
 int pair_threads(int v) { return v >= 0 && v < kNumPair ? 2 * kPairNV[v] : 0; }
 
 int pair_txmax(int N, int v) {
