@@ -453,7 +453,8 @@ int run_coupled(fomo_ctx* ctx, const fomo_grid2d* gp, const float* vp, const flo
   // runs that fit keep their state on the chip (resident2d.cuh): 400x300 with nbc 100
   // 15.0 -> 9.7 us per step
   res::Plan rp;
-  if (on_chip && nt > res::kMinSteps && !(opts && (opts->flags & FOMO_F_STEP_LAUNCH)))
+  if (on_chip && nt > res::kMinSteps && !(opts && (opts->flags & FOMO_F_STEP_LAUNCH)) &&
+      (!opts || opts->kernel == FOMO_KERNEL_AUTO))
     rp = res::make_plan(res::kCoupledNeeds, N, g.nx, g.nz, g.ld, g.nbc, 1,
                         res::sm_count(ctx->device), res::smem_extra(hhp.wstride, 0));
   if (rp.ok) res::plan_entries(rp, 1, tags);

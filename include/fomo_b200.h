@@ -70,10 +70,12 @@ extern "C" {
 #define FOMO_BF16 2
 
 /* fomo_opts.kernel: time-step kernel family (0 lets the autotuner pick) */
-#define FOMO_KERNEL_AUTO 0
-#define FOMO_KERNEL_TWO_PHASE 1    /* velocity sweep + stress sweep per step; runs of */
-                                   /* more than 300 steps on grids that fit on chip   */
-                                   /* are one cooperative launch of the same updates  */
+#define FOMO_KERNEL_AUTO 0         /* 2D FP32 runs of more than 300 steps on grids      */
+                                   /* that fit on the chip are one cooperative launch  */
+                                   /* of the two-phase updates (stats: TWO_PHASE, and  */
+                                   /* alg_bytes as if launched: the state stays on the */
+                                   /* chip)                                            */
+#define FOMO_KERNEL_TWO_PHASE 1    /* velocity sweep + stress sweep per step, launched */
 #define FOMO_KERNEL_SINGLE_SWEEP 2 /* one fused sweep per step (z-marching tiles); */
                                    /* 3D: two TMA-staged half steps per step, each    */
                                    /* with its Higdon boundary fused (AUTO's pick,    */

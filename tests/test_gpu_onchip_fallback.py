@@ -66,6 +66,26 @@ def test_failed_run_on_chip_is_launched(fomo, monkeypatch, name, flag):
         assert np.isfinite(a).all() and np.abs(a).max() > 0
 
 
+@pytest.mark.parametrize("name", ["acoustic2d", "elastic2d", "scalar2d", "coupled2d"])
+def test_two_phase_is_launched(fomo, monkeypatch, name):
+    """FOMO_KERNEL_TWO_PHASE asks for launched steps; only AUTO keeps a run on the chip."""
+    from fomo_b200 import _lib as L
+
+    orig, got = fomo.api._opts, []
+    for kernel in (L.FOMO_KERNEL_AUTO, L.FOMO_KERNEL_TWO_PHASE):
+        def opts(*a, kernel=kernel, **kw):
+            o = orig(*a, **kw)
+            o.kernel = kernel
+            return o
+
+        monkeypatch.setattr(fomo.api, "_opts", opts)
+        fin, fn = _calls(fomo)[name]()
+        got.append((_flat(fn(**fin), fin), fomo.api.last_stats.gpu_launches))
+    assert got[0][1] <= 16 and got[1][1] > NT
+    for a, b in zip(got[0][0], got[1][0]):
+        assert np.array_equal(a, b)
+
+
 def test_two_contexts_on_chip_at_once(fomo, monkeypatch):
     """Two threads with a context each: every run wants one CTA per SM."""
     from fomo_b200 import _lib as L
