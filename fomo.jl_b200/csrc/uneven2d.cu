@@ -1141,7 +1141,9 @@ int run_uneven(fomo_ctx* ctx, float dh, float dt, int nt, int nbc, int fd_order,
   }
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
-  if (use_bulk) {  // chunks of 32 steps captured once and replayed, the rest launched
+  constexpr int K = 32;  // steps of a replayed chunk
+  const int nchunk = use_bulk && nt >= 2 * K ? nt / K : 0;
+  if (use_bulk) {  // chunks of K steps captured once and replayed, the rest launched
     BShot* d_bs = ws_ptr<BShot>(ctx, o_bshot);
     int* d_bblk = ws_ptr<int>(ctx, o_bblk);
     int* d_it = ws_ptr<int>(ctx, o_it);
@@ -1161,8 +1163,6 @@ int run_uneven(fomo_ctx* ctx, float dh, float dt, int nt, int nbc, int fd_order,
       k_uinject_record<<<ns, 256, 0, s2>>>(d_tab, d_state, d_src, d_wav, d_rec, d_seis, it, nt,
                                            1 - A, it0);
     };
-    constexpr int K = 32;
-    const int nchunk = nt >= 2 * K ? nt / K : 0;
     if (nchunk) {
       cudaStream_t cs2 = ctx->own_stream;  // the caller's stream may be uncapturable
       FOMO_CU(ctx, cudaStreamBeginCapture(cs2, cudaStreamCaptureModeThreadLocal));
@@ -1232,7 +1232,7 @@ int run_uneven(fomo_ctx* ctx, float dh, float dt, int nt, int nbc, int fd_order,
     // acoustic: vx, vz, p read and written + bx, bz, kappa read = 9 words per cell
     stats->alg_bytes = 36.0 * (double)cells * nt;
     stats->n_shots = ns;
-    stats->gpu_launches = fused ? 1 : 3 * nt;
+    stats->gpu_launches = fused ? 1 : 3 * nt + nchunk;  // + each chunk's step counter
     stats->kernel = fused ? FOMO_KERNEL_SINGLE_SWEEP : FOMO_KERNEL_TWO_PHASE;
     stats->sweep_config = fused ? kAcNTX[a_k] * 1000 : t.bx * 1000 + t.by;
   }

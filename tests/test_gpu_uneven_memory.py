@@ -1,4 +1,5 @@
-"""Device memory of the uneven batch: nine padded planes a shot and its acquisition."""
+"""Device memory of the uneven batch (nine padded planes a shot and its acquisition) and the
+launches it counts."""
 import numpy as np
 import pytest
 
@@ -34,3 +35,12 @@ def test_models_are_staged_in_the_state(fomo, monkeypatch, kernel):
         for a, b in zip(x, y):
             assert np.array_equal(a, b)
             assert np.abs(a).max() > 0
+
+
+@pytest.mark.parametrize("nt,chunks", [(63, 0), (64, 2), (100, 3)])
+def test_launches_counted(fomo, nt, chunks):
+    """Three launches a step, and a step counter per replayed chunk of 32 steps."""
+    vp = np.full((40, 31), 2500, np.float32, order="F")
+    fomo.acoustic2d_uneven([vp, vp], [vp, vp], 10.0, 1e-3, nt, 15.0, sx=[[9]] * 2, sz=[[9]] * 2,
+                           rx=[[3]] * 2, rz=[[4]] * 2, nbc=5)
+    assert fomo.api.last_stats.gpu_launches == 3 * nt + chunks
