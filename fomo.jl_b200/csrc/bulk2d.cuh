@@ -23,7 +23,8 @@ constexpr int kW = 128;  // columns of an inner tile: a warp of 4-cell threads
 constexpr int kThreads = 256;
 // CTAs per SM that the acoustic kernels' registers are bounded to: without the bound
 // (2 to 3) too few loads are in flight to cover the latency (64 uneven
-// shots 466 us per step, with 4 349, with 5, which spills, 372).
+// shots 466 us per step, with 4 349, with 5 372).  At 4 some forms spill a few words (8 to 12
+// bytes untagged, the tagged order-8 pressure kernel 96 / 104), at 5 all of them many.
 constexpr int ac_blocks(int N) { return N <= 4 ? 4 : 3; }
 
 // The inner rectangle [x0, x1) x [z0, z1) (x0, x1 multiples of 4), its tiles, and the

@@ -19,11 +19,17 @@
 // second on the global timer, recorded in *err); after that the tile stops waiting,
 // and the host runs the steps again as launches, which wait for nobody.
 //
-// What it measured (us per step, order 8, this form / replayed two-phase launches):
-// acoustic 240x200 nbc 50 4.7 / 9.1, 400x300 nbc 100 5.9 / 12.8, 4 shots of 240x200
-// 7.4 / 14.9, eight 13.2 / 22.9, 1000x800 12.9 / 21.7 (materials from L2); elastic 240x200 6.7 / 10.5, 501x397 10.9 / 17.0; scalar 240x200 2.1 / 4.1,
-// 500x400 2.8 / 5.6, 1000x800 5.3 / 10.5; coupled 400x300 nbc 100 9.7 / 15.0.  An exchange costs about 0.7 us, the rest is issue and latency of the
-// phases between barriers (36 % issue active at 20 warps per SM).
+// What it measured (us per step, order 8, nbc 50 where none is given, this form / replayed
+// two-phase launches, in blocks per thread from 200 k inner cells):
+// acoustic 240x200 4.5 / 8.0, 400x300 nbc 100 6.0 / 12.3, 4 shots of 240x200 7.6 / 14.2,
+// eight 13.2 / 18.7, 1000x800 12.6 / 14.1 (materials from L2); elastic 240x200 6.3 / 9.4,
+// 501x397 10.4 / 16.1, 640x560 nbc 20 12.5 / 14.0; scalar 240x200 2.1 / 3.6, 500x400 2.7 / 5.1,
+// 1000x800 5.5 / 6.1; coupled 400x300 nbc 100 10.2 / 13.4.  It is the faster form up to the
+// largest grids that fit, at order 10 too.  With the updates taken out, the exchange and the
+// barriers alone take 1.3 of the 2.1 us of a scalar step and, for its two exchanges, 2.6 of
+// the 4.5 us of an acoustic step (240x200; 4.1 of 12.6 at 1000x800).  The rest is issue and
+// latency of the phases between barriers: 46 to 49 % of the issue slots are used, at 20
+// warps per SM (30 for scalar 240x200), by more integer than floating point instructions.
 //
 // A tile computes its own cells and a one-cell ring around them (the inward
 // neighbours of the Higdon terms), so the ring's old values come with the halo and the
@@ -614,8 +620,9 @@ struct Plan {
 struct Needs {
   int hal, ext, mats, mreg, strips, bands, rows, cols;
   int wide;  // strips and bands are 2N + 1 + wide cells wide in all
-  int forms; // block forms in use: 4 x 4 blocks of the elastic and coupled updates spill
-             // (elastic 700x600 30.2 us per step against 23.2 launched)
+  int forms; // block forms in use: the elastic and coupled updates spill some words in
+             // every form (52 / 96 bytes stored / loaded at 4 x 1, order 8), in 4 x 4 blocks
+             // so many that launches are faster (elastic 700x600 30.2 us per step against 23.2)
 };
 constexpr Needs kAcousticNeeds{3, 2, 3, 8, 2, 2, 1, 1, 0, 4};
 constexpr Needs kElasticNeeds{5, 3, 5, 0, 4, 4, 1, 1, 0, 3};
@@ -638,9 +645,12 @@ struct Tables {
 Tables take_tables(Arena& ar, const Plan& p);
 cudaError_t upload_tables(cudaStream_t st, char* ws, const Plan& p, const Tables& t,
                           const CellTags& tags, Run& run);
-// Runs of more steps than this keep their state on the chip when it fits: at every
-// size measured that halves the step.  Shorter runs gain under 2 ms a call and keep the
-// replayed launches, whose count callers read in the stats and the tests pin.
+// Runs of more steps than this keep their state on the chip when it fits.  The line is
+// not where the time turns: on chip a call is the faster one from 10 to 50 steps on (call
+// ms, on chip / launched, at 50, 100 and 300 steps: acoustic 400x300 nbc 100 0.7 / 1.2,
+// 1.1 / 2.0, 2.4 / 4.7; 1000x800 2.0 / 2.1, 2.7 / 2.9, 5.4 / 6.2; elastic 501x397 1.1 / 1.5,
+// 1.7 / 2.6, 3.9 / 5.9; coupled 400x300 1.0 / 1.3, 1.6 / 2.2, 3.7 / 5.1).  Up to here runs keep
+// the replayed launches, whose number callers read in the stats and tests fix at 300 steps.
 constexpr int kMinSteps = 300;
 int sm_count(int device);
 
