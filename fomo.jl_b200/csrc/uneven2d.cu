@@ -1057,7 +1057,9 @@ int run_uneven(fomo_ctx* ctx, float dh, float dt, int nt, int nbc, int fd_order,
       auto it = g_utune.find(key);
       if (it != g_utune.end()) pin = it->second;
     }
-    if (pin < 0) {  // time each strip width on three steps of the zero state
+    // Time each strip width on up to three steps of the zero state.  The launch injects and
+    // records, and wavelets and seismograms hold nt steps: never more than those.
+    if (pin < 0) {
       FOMO_CU(ctx, cudaMemsetAsync(d_state, 0, 4 * off_state, st));
       float best = 1e30f;
       for (int k = 0; k < kAcNumNTX; ++k) {
@@ -1066,7 +1068,7 @@ int run_uneven(fomo_ctx* ctx, float dh, float dt, int nt, int nbc, int fd_order,
         a_k = k;
         FOMO_CU(ctx, ac_run(st, 1, 1));
         FOMO_CU(ctx, cudaEventRecord(ctx->ev0, st));
-        FOMO_CU(ctx, ac_run(st, 1, 3));
+        FOMO_CU(ctx, ac_run(st, 1, std::min(3, nt)));
         FOMO_CU(ctx, cudaEventRecord(ctx->ev1, st));
         FOMO_CU(ctx, cudaEventSynchronize(ctx->ev1));
         float ms = 0.0f;
